@@ -37,14 +37,16 @@
 
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 
 #include "beep_internal.h"
+#include "rng_filter.cuh"
 #include "rng_fp64.cuh"
 
 namespace beep {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kMaxThreads = 512;
 
 __device__ double normal_lp(double x, double mean, double var)
 {
@@ -137,28 +139,90 @@ __device__ void democat_adjust(const ModelDev &m, double *pop, int sett, int tid
 	}
 }
 
-// PopT: int32_t, or double for models with demographic changes
+// n / d for the kernel's index splits: one multiply where every n in [0, nmax] allows it
+struct Div {
+	uint32_t d, mul;
+	__device__ __forceinline__ Div(int div, size_t nmax) : d((uint32_t)div), mul(0u)
+	{
+		if (d > 1 && (unsigned long long)nmax * d < 0x100000000ull) mul = 0xffffffffu / d + 1u;
+	}
+	__device__ __forceinline__ int quot(int n) const
+	{
+		return d == 1 ? n : mul ? (int)__umulhi((uint32_t)n, mul) : (int)((uint32_t)n / d);
+	}
+};
+
+// FP64 values tested on the integer pipe
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ bool is_nan(double x)
+{
+	return (unsigned long long)(__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ull;
+}
+
+// What the kernel keeps in shared memory: level 2 the particle's arrays and the tables, level 1
+// the tables (a larger model's arrays stay in its global work region), level 0 nothing.
+// The step's tables are double-buffered: a step's are loaded during the previous step's draws.
+struct PlainSmem {
+	size_t pop, tn, imap, idiag, dinf, x, rate, sus, infdif, bea, eta, N, diag, fac, from, to, age, adp, brow, eref, total;
+	__host__ __device__ PlainSmem(const ModelDev &m, int pop_bytes, int level)
+	{
+		size_t off = 0;
+		const bool state = level == 2;
+		auto take = [&](size_t n) { const size_t o = off; off += level == 0 ? 0 : (n + 15) & ~(size_t)15; return o; };
+		const size_t ncol = (size_t)m.A * m.DP, ag = (size_t)m.NS * m.A * m.G, sa = (size_t)m.NS * m.A;
+		pop = take(state ? 2 * (size_t)pop_bytes * m.C * ncol : 0);
+		tn = take(state ? 4 * (size_t)m.T * ncol : 0);
+		imap = take(state ? 8 * ag : 0);
+		idiag = take(state ? 8 * ag : 0);
+		dinf = take(state ? 8 * ag : 0);
+		x = take(state ? 8 * ag : 0);
+		rate = take(8 * (size_t)m.T * m.DP);
+		sus = take(8 * (size_t)m.DP);
+		infdif = take(8 * (size_t)m.T);
+		bea = take(16 * sa);
+		eta = take(16 * sa);
+		N = take(16 * (size_t)m.G * m.G);
+		diag = take(8 * (size_t)m.A);
+		fac = take(8 * (size_t)m.A);
+		from = take(4 * (size_t)m.T);
+		to = take(4 * (size_t)m.T);
+		age = take(4 * (size_t)m.DPS);
+		adp = take(4 * (size_t)m.G);
+		brow = take(4 * sa);
+		eref = take(4 * sa);
+		total = off;
+	}
+};
+
+// One CTA per particle.  Bound: latency of a step's dependent phases for small models; the
+// FP64 pipe (one warp instruction per 16 cycles and SM) for large ones, where the
+// area-mixing sums, two operations per (source, target, age), remain.  Everything else
+// was taken off that pipe: the draws are decided in FP32 (rng_filter.cuh), comparisons and
+// zero tests are done on the bits, a target's NMI terms are formed once instead of once
+// per age, unit observation factors sum their integer counts as integers.
+// PopT: int32_t, or double for models with demographic changes.
 template <typename PopT>
-__global__ void __launch_bounds__(kThreads) sim_plain_kernel(const ModelDev m, const BatchDev b)
+__global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m, const BatchDev b, const int level)
 {
 	constexpr bool kPop64 = sizeof(PopT) == 8;
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	__shared__ FilterTab ftab;
 	const uint32_t lim = b.sampler_limit ? b.sampler_limit : 65536u;   // sampler rejection iterations
 	const int p = blockIdx.x;
 	if (p >= b.P) return;
 	const int tid = threadIdx.x, nth = blockDim.x;
-	const int A = m.A, G = m.G, DP = m.DP, NS = m.NS, DPS = m.DPS, C = m.C, T = m.T;
-	const size_t popsz = (size_t)A * C * DP, tnsz = (size_t)A * T * DP, agsz = (size_t)NS * A * G;
+	const int A = m.A, G = m.G, DP = m.DP, NS = m.NS, DPS = m.DPS, C = m.C, T = m.T, ncol = A * DP, GG = G * G;
+	const size_t popsz = (size_t)C * ncol, tnsz = (size_t)T * ncol;
+	const int agsz = NS * A * G, NSA = NS * A;
 	const int nsteps = b.tf - b.ti;
 	const GroupDir dir = b.dirs[b.group_of ? b.group_of[p] : 0];
 	const uint32_t stream = b.stream_of ? b.stream_of[p] : (uint32_t)p;
 	const uint32_t k0 = b.key_of ? b.key_of[p].x : b.k0, k1 = b.key_of ? b.key_of[p].y : b.k1;   // the particle's key
 	const double *fp = b.fpool;
 	const int32_t *ip = b.ipool;
-	const double *transrate = fp + dir.transrate, *sus = fp + dir.susceptibility, *infectivity = fp + dir.infectivity;
-	const double *infdif = fp + dir.infdif, *beta_rows = fp + dir.beta_rows, *areafactor = fp + dir.areafactor;
+	const double *infectivity = fp + dir.infectivity, *beta_rows = fp + dir.beta_rows, *areafactor = fp + dir.areafactor;
 	const double *Ntime = fp + dir.Ntime, *geo = fp + dir.geo_spline, *efoi_spline = fp + dir.efoi_spline;
 	const double *efoi_age = fp + dir.efoi_agedist, *obs_spline = fp + dir.obs_spline;
-	const int32_t *beta_row_of = ip + dir.beta_row_of, *efoi_ref = ip + dir.efoi_ref;
 	const double *efoi_mult = dir.efoi_mult >= 0 ? fp + dir.efoi_mult : nullptr;
 	const double *tm_mult = dir.tm_mult >= 0 ? fp + dir.tm_mult : nullptr;
 
@@ -170,122 +234,163 @@ __global__ void __launch_bounds__(kThreads) sim_plain_kernel(const ModelDev m, c
 	auto chs = [&](int slot, int s) { return ((size_t)slot * b.P + p) * m.S + s; };
 	double Lsum = 0.0, Lcmp = 0.0;   // mode 2: compensated partial sum of this thread
 
-	PopT *pop_cur = (PopT *)b.pop_a + (size_t)p * popsz;
-	PopT *pop_nxt = (PopT *)b.pop_b + (size_t)p * popsz;
-	double *Imap = b.Imap + (size_t)p * agsz, *Idiag = b.Idiag + (size_t)p * agsz;
-	double *dinf = b.dinf + (size_t)p * agsz, *NMI = b.NMI + (size_t)p * agsz;
+	const bool smem_state = level == 2, smem_tabs = level >= 1;
+	const PlainSmem lay(m, (int)sizeof(PopT), level);
+	PopT *pop_cur = smem_state ? (PopT *)(smem_raw + lay.pop) : (PopT *)b.pop_a + (size_t)p * popsz;
+	PopT *pop_nxt = smem_state ? pop_cur + popsz : (PopT *)b.pop_b + (size_t)p * popsz;
+	double *Imap = smem_state ? (double *)(smem_raw + lay.imap) : b.Imap + (size_t)p * agsz;
+	double *Idiag = smem_state ? (double *)(smem_raw + lay.idiag) : b.Idiag + (size_t)p * agsz;
+	double *dinf = smem_state ? (double *)(smem_raw + lay.dinf) : b.dinf + (size_t)p * agsz;
+	double *X = smem_state ? (double *)(smem_raw + lay.x) : b.NMI + (size_t)p * agsz;   // NMI terms (NMI for one age)
 	double *acc = b.obs_acc + (size_t)p * b.nscored;
+	double *bea = (double *)(smem_raw + lay.bea), *eta = (double *)(smem_raw + lay.eta), *Nm = (double *)(smem_raw + lay.N);
+	int32_t *adp = (int32_t *)(smem_raw + lay.adp);      // the dp of each age, where each has one
+	const bool one_dp = smem_tabs && m.dp_age_unique;
 	int32_t *status = b.status + p;
 
 	for (size_t k = tid; k < popsz; k += nth)
 		pop_cur[k] = b.ti == 0 ? (PopT)m.pop_init[k] : ((const PopT *)b.pop_in)[(size_t)p * popsz + k];
 	for (int k = tid; k < b.nscored; k += nth) acc[k] = 0.0;
+	// tables in shared memory (level >= 1) or where they are
+	auto table = [&](size_t off, const auto *src, int n) {
+		if (!smem_tabs) return src;
+		auto *dst = (std::remove_const_t<std::remove_pointer_t<decltype(src)>> *)(smem_raw + off);
+		for (int k = tid; k < n; k += nth) dst[k] = src[k];
+		return (decltype(src))dst;
+	};
+	const double *rate = table(lay.rate, fp + dir.transrate, T * DP), *sus = table(lay.sus, fp + dir.susceptibility, DP);
+	const double *infdif = table(lay.infdif, fp + dir.infdif, T);
+	const double *diag = table(lay.diag, m.M_diag, A), *afac = table(lay.fac, m.M_factor, A);
+	const int32_t *from = table(lay.from, m.trans_from, T), *to = table(lay.to, m.trans_to, T);
+	const int32_t *age = table(lay.age, m.dp_age, DPS);
+	const int32_t *brow = table(lay.brow, ip + dir.beta_row_of, NSA), *eref = table(lay.eref, ip + dir.efoi_ref, NSA);
+	if (one_dp)
+		for (int dp = tid; dp < DPS; dp += nth) adp[m.dp_age[dp]] = dp;
+	filter_tab_fill(ftab, tid, nth);
 	__syncthreads();
+
+	const Div divDP(DP, tnsz + popsz), divG(G, agsz), divA(A, NSA), divDPS(DPS, (size_t)A * DPS);
+	// a step's tables of (strain, area) i: beta * areafactor, external force per capita
+	auto slice = [&](int s, int i, double &be, double &et) {
+		const int st = divA.quot(i), c = i - st * A;
+		be = beta_rows[(size_t)brow[i] * m.S + s] * areafactor[(size_t)(s / m.div_per_time) * A + c];
+		et = efoi_spline[(size_t)eref[i] * m.S + s];
+		if (!is_zero(et)) et = et / m.popsize;
+		if (efoi_mult) et *= efoi_mult[((size_t)s * A + c) * NS + st];
+	};
+	for (int i = tid; smem_tabs && i < NSA; i += nth) slice(b.ti, i, bea[i], eta[i]);
+	for (int i = tid; smem_tabs && i < GG; i += nth) Nm[i] = Ntime[(size_t)b.ti * GG + i];
+
+	// draws of a step: (transition, column), the columns of a transition padded to whole warps
+	// where that costs no further pass of the CTA (a warp then draws from similar means)
+	const int pad = (ncol + 31) & ~31;
+	const int cols = (T * pad + nth - 1) / nth <= ((int)tnsz + nth - 1) / nth ? pad : ncol;
+	const Div divCol(cols, (size_t)T * cols);
+	// dinf per (strain, source area, age) of the next step's maps, from the step's counts
+	auto dinf_of_counts = [&](const int32_t *cnt, const int32_t *base) {
+		for (int idx = tid; idx < agsz; idx += nth) {
+			const int sc = divG.quot(idx), a = idx - sc * G, st = divA.quot(sc), c = sc - st * A;
+			double s = 0.0;
+			for (int tr = 0; tr < T; tr++) {
+				const double di = infdif[tr];
+				if (is_zero(di)) continue;
+				const int dp0 = one_dp ? adp[a] : 0, dp1 = one_dp ? dp0 + 1 : DPS;
+				for (int dp = dp0; dp < dp1; dp++) {
+					if (age[dp] != a) continue;
+					const int cl = (c * T + tr) * DP + st * DPS + dp;
+					const int num = base ? cnt[cl] - base[cl] : cnt[cl];
+					if (num != 0) s += di * (double)num;
+				}
+			}
+			dinf[idx] = s;
+		}
+	};
 
 	const int itr = m.infection_trans;
 	const int inf_from = m.trans_from[itr];
+	int buf = 0;
+	int opos = b.step_ptr[0] + tid < b.step_ptr[1] ? b.step_obs[b.step_ptr[0] + tid] : 0;   // this thread's first observation
 	for (int sett = b.ti; sett < b.tf; sett++) {
-		int32_t *tn = mode ? b.ch_tn + chs(writes ? cs_p : cs_i, sett) * tnsz
-		          : b.tn_traj ? b.tn_traj + ((size_t)p * nsteps + (sett - b.ti)) * tnsz : b.tn + (size_t)p * tnsz;
-		const int32_t *tn_prev = b.tn_traj || mode ? tn - tnsz : tn;   // single buffer still holds the previous step
-		const int32_t *tn_base = dif && sett > 0 ? b.ch_tn + chs(cs_i, sett - 1) * tnsz : nullptr;
-		double *Im_s = mode ? b.ch_Imap + chs(writes ? cs_p : cs_i, sett) * agsz : Imap;
-		double *Id_s = mode ? b.ch_Idiag + chs(writes ? cs_p : cs_i, sett) * agsz : Idiag;
+		// the step's counts: in shared memory, or the output or chain array itself (ext)
+		int32_t *ext = mode ? b.ch_tn + chs(writes ? cs_p : cs_i, sett) * tnsz
+		           : b.tn_traj ? b.tn_traj + ((size_t)p * nsteps + (sett - b.ti)) * tnsz : nullptr;
+		int32_t *tn = smem_state ? (int32_t *)(smem_raw + lay.tn) : ext ? ext : b.tn + (size_t)p * tnsz;
+		const bool copy = smem_state && ext;
+		const double *be = bea + buf * NSA, *et = eta + buf * NSA;
+		const double *N = smem_tabs ? Nm + buf * GG : Ntime + (size_t)sett * GG;
+		const int sn = sett + 1 < b.tf ? sett + 1 : sett;
+		const double d = geo[sett], omd = 1 - d;
+		const int s0 = b.step_ptr[sett - b.ti], s1 = mode == 2 ? s0 : b.step_ptr[sett - b.ti + 1];
+		const int oidx = s0 + tid < s1 ? b.scored[opos] : -1;
 
 		if constexpr (kPop64) {
 			if (m.ndcc > 0) democat_adjust(m, pop_cur, sett, tid, nth);   // pop[sett] before its step
 		}
-
-		// ---- A: dinf per (strain, source area, age)
-		for (int idx = tid; idx < (int)agsz && mode != 2 && !(dif && sett == 0); idx += nth) {
-			const int a = idx % G, c = (idx / G) % A, st = idx / (G * A);
-			double s = 0.0;
-			if (sett == b.ti) {
+		if (sett == b.ti && mode != 2 && !dif) {
+			// the start populations' infectious counts
+			for (int idx = tid; idx < agsz; idx += nth) {
+				const int sc = divG.quot(idx), a = idx - sc * G, st = divA.quot(sc), c = sc - st * A;
+				double s = 0.0;
 				for (int co = 0; co < C; co++) {
 					const double inf = infectivity[co];
 					if (inf != 0) {
 						for (int dp = 0; dp < DPS; dp++) {
-							if (m.dp_age[dp] != a) continue;
+							if (age[dp] != a) continue;
 							const double pv = (double)pop_cur[((size_t)c * C + co) * DP + st * DPS + dp];
 							if (pv != 0) s += inf * pv;
 						}
 					}
 				}
+				dinf[idx] = s;
+			}
+			__syncthreads();
+		}
+
+		// ---- B: Imap/Idiag per (strain, target area, age), sources in ascending order, and
+		// the target's NMI term (INF_DIF_UPDATE: the running sums are dImap/dIdiag and the
+		// state's maps are the current state's plus them); strain shift of the susceptibles
+		for (int idx = tid; idx < agsz; idx += nth) {
+			const int sc = divG.quot(idx), a = idx - sc * G, st = divA.quot(sc), t = sc - st * A;
+			double imv, idv;                               // the state's maps
+			const size_t io = mode ? chs(cs_i, sett) * agsz + idx : 0;
+			if (mode == 2) {
+				imv = b.ch_Imap[io];
+				idv = b.ch_Idiag[io];
 			} else {
-				for (int tr = 0; tr < T; tr++) {
-					const double di = infdif[tr];
-					if (di != 0) {
-						for (int dp = 0; dp < DPS; dp++) {
-							if (m.dp_age[dp] != a) continue;
-							const size_t cl = ((size_t)c * T + tr) * DP + st * DPS + dp;
-							const double num = tn_base ? (double)(tn_prev[cl] - tn_base[cl]) : (double)tn_prev[cl];
-							if (num != 0) s += di * num;
-						}
+				const double *dst = dinf + (size_t)st * A * G + a;
+				double im = sett == b.ti ? 0.0 : Imap[idx];
+				double id = sett == b.ti ? 0.0 : Idiag[idx];
+				if (!(dif && sett == b.ti)) {
+					const double dself = dst[t * G];
+					if (!is_zero(dself)) id += dself * diag[t];
+					const int j1 = m.csc_ptr[t + 1];
+#pragma unroll 4
+					for (int j = m.csc_ptr[t]; j < j1; j++) {
+						const double ds = dst[m.csc_src[j] * G], v = m.csc_val[j];
+						if (!is_zero(ds)) im += ds * v;
 					}
 				}
-			}
-			dinf[idx] = s;
-		}
-		__syncthreads();
-
-		// ---- B: Imap/Idiag per (strain, target area, age), sources in ascending order
-		// (INF_DIF_UPDATE: the running sums are dImap/dIdiag and the state's maps
-		// are the current state's plus them)
-		for (int idx = tid; idx < (int)agsz && mode != 2; idx += nth) {
-			const int a = idx % G, t = (idx / G) % A, st = idx / (G * A);
-			const double *dst = dinf + (size_t)st * A * G;
-			double im = sett == b.ti ? 0.0 : Imap[idx];
-			double id = sett == b.ti ? 0.0 : Idiag[idx];
-			if (!(dif && sett == 0)) {
-				const double dself = dst[t * G + a];
-				if (dself != 0) id += dself * m.M_diag[t];
-				for (int j = m.csc_ptr[t]; j < m.csc_ptr[t + 1]; j++) {
-					const double d = dst[m.csc_src[j] * G + a];
-					if (d != 0) im += d * m.csc_val[j];
+				Imap[idx] = im;
+				Idiag[idx] = id;
+				imv = dif ? b.ch_Imap[io] + im : im;
+				idv = dif ? b.ch_Idiag[io] + id : id;
+				if (writes) {
+					const size_t ow = chs(cs_p, sett) * agsz + idx;
+					b.ch_Imap[ow] = imv;
+					b.ch_Idiag[ow] = idv;
 				}
 			}
-			Imap[idx] = im;
-			Idiag[idx] = id;
-			if (writes) {
-				if (dif) {
-					const size_t io = chs(cs_i, sett) * agsz + idx;
-					Im_s[idx] = b.ch_Imap[io] + im;
-					Id_s[idx] = b.ch_Idiag[io] + id;
-				} else {
-					Im_s[idx] = im;
-					Id_s[idx] = id;
-				}
-			}
-		}
-		__syncthreads();
-
-		// ---- C: NMI per (strain, area, age); strain shift of the susceptible population
-		for (int idx = tid; idx < (int)agsz; idx += nth) {
-			const int a = idx % G, c = (idx / G) % A, st = idx / (G * A);
-			const double *Id = Id_s + (size_t)st * A * G, *Im = Im_s + (size_t)st * A * G;
-			const double d = geo[sett];
-			const double omd = 1 - d;
-			const double fac = m.M_factor[c];
-			double val;
+			const double fac = afac[t];
 			if (G == 1) {
-				val = Id[c] * (d + fac * omd) + Im[c] * d;
-				if (val < 0) val = 0;
+				const double val = idv * (d + fac * omd) + imv * d;
+				X[idx] = val < 0 ? 0 : val;
 			} else {
-				const int v = c * G;
-				const double *N = Ntime + ((size_t)sett * G + a) * G;
-				double sum = 0.0;
-				for (int aa = 0; aa < G; aa++) {
-					const double I = (Id[v + aa] + Im[v + aa]) * d + fac * Id[v + aa] * omd;
-					sum += N[aa] * I;
-				}
-				if (sum < 0) sum = 0;
-				val = sum;
+				X[idx] = (idv + imv) * d + fac * idv * omd;
 			}
-			NMI[idx] = val;
 		}
 		if (NS > 1) {
 			for (int idx = tid; idx < A * DPS; idx += nth) {
-				const int dp = idx % DPS, c = idx / DPS;
+				const int c = divDPS.quot(idx), dp = idx - c * DPS;
 				PopT *sp = pop_cur + ((size_t)c * C + inf_from) * DP;
 				double sum = 0.0;
 				for (int st = 1; st < NS; st++) {
@@ -298,124 +403,180 @@ __global__ void __launch_bounds__(kThreads) sim_plain_kernel(const ModelDev m, c
 		}
 		__syncthreads();
 
-		// ---- D: transition means and counts per (area, transition, dp)
-		for (int cell = tid; cell < (int)tnsz; cell += nth) {
-			const int dp = cell % DP, tr = (cell / DP) % T, c = cell / (DP * T);
-			double mean;
+		// ---- D: transition means and counts per (transition, column); the next step's tables
+		// and this thread's next observation are loaded on the way
+		double nbe = 0.0, net = 0.0, nN = 0.0;
+		if (smem_tabs && tid < NSA) slice(sn, tid, nbe, net);
+		if (smem_tabs && tid < GG) nN = Ntime[(size_t)sn * GG + tid];
+		int oq0 = 0, oq1 = 0, ospl = -1;
+		double ofac = 0.0, oacc = 0.0;
+		if (oidx >= 0) {
+			oq0 = m.obs_cell_ptr[oidx];
+			oq1 = m.obs_cell_ptr[oidx + 1];
+			ospl = m.obs_spline[oidx];
+			ofac = m.obs_factor[oidx];
+			oacc = acc[opos];
+		}
+		const int s2 = sett + 1 < b.tf && mode != 2 ? b.step_ptr[sett + 2 - b.ti] : s1;
+		const int npos = s1 + tid < s2 ? b.step_obs[s1 + tid] : 0;
+		for (int item = tid; item < T * cols; item += nth) {
+			const int tr = divCol.quot(item), col = item - tr * cols;
+			if (col >= ncol) continue;
+			const int c = divDP.quot(col), dp = col - c * DP;
+			const size_t cell = ((size_t)c * T + tr) * DP + dp;
+			double mean = 0.0;
 			if (tr == itr) {
-				const int st = dp / DPS, dpl = dp % DPS;
-				const double popu = (double)pop_cur[((size_t)c * C + inf_from) * DP + dpl];
-				if (popu <= 0) mean = 0;
-				else {
-					const int a = m.dp_age[dpl];
-					double be = beta_rows[(size_t)beta_row_of[st * A + c] * m.S + sett];
-					be *= areafactor[(size_t)(sett / m.div_per_time) * A + c];
-					const int ei = efoi_ref[st * A + c];
-					double et = efoi_spline[(size_t)ei * m.S + sett] / m.popsize;
-					if (efoi_mult) et *= efoi_mult[((size_t)sett * A + c) * NS + st];
-					const double eta = et * efoi_age[(size_t)ei * G + a];
-					mean = m.dt * popu * sus[dp] * (be * NMI[((size_t)st * A + c) * G + a] + eta);
+				const int st = dp / DPS, dpl = dp - st * DPS;
+				const PopT popu = pop_cur[((size_t)c * C + inf_from) * DP + dpl];
+				if (popu > 0) {
+					const int sc = st * A + c, a = age[dpl];
+					double nmi;
+					if (G == 1) nmi = X[sc];
+					else {
+						nmi = 0.0;
+						for (int aa = 0; aa < G; aa++) nmi += N[a * G + aa] * X[sc * G + aa];
+						if (nmi < 0) nmi = 0;
+					}
+					double bsc, esc;
+					if (smem_tabs) { bsc = be[sc]; esc = et[sc]; }
+					else slice(sett, sc, bsc, esc);
+					const double ext_foi = esc * efoi_age[(size_t)eref[sc] * G + a];
+					mean = m.dt * (double)popu * sus[dp] * (bsc * nmi + ext_foi);
 				}
 			} else {
-				const double popu = (double)pop_cur[((size_t)c * C + m.trans_from[tr]) * DP + dp];
-				mean = popu <= 0 ? 0 : m.dt * popu * transrate[(size_t)tr * DP + dp];
+				const PopT popu = pop_cur[((size_t)c * C + from[tr]) * DP + dp];
+				if (popu > 0) mean = m.dt * (double)popu * rate[tr * DP + dp];
 			}
 			if (tm_mult) mean *= tm_mult[(size_t)sett * tnsz + cell];   // prediction modifications
-			if (mode == 2) {                    // State::likelihood term of the fixed count
-				if (mean != mean) set_status(status, BEEP_NAN_RATE);
-				const double lp = poisson_lp(tn[cell], mean);
-				const double t = Lsum + lp;
-				Lcmp += fabs(Lsum) >= fabs(lp) ? (Lsum - t) + lp : (lp - t) + Lsum;
-				Lsum = t;
-				continue;
-			}
-			if (mode == 3) {                    // the given counts stay
-				if (mean != mean) set_status(status, BEEP_NAN_RATE);
-				b.ch_mean[chs(cs_p, sett) * tnsz + cell] = mean;
-				continue;
-			}
+			const bool bad = is_nan(mean);
+			if (bad) set_status(status, BEEP_NAN_RATE);
 			int32_t n = 0;
-			if (mean != mean) set_status(status, BEEP_NAN_RATE);
-			else if (mean != 0) {
-				if (mean > 1000000000.0) set_status(status, BEEP_COUNT_OVERFLOW);
+			if (mode >= 2) {                    // the given counts stay
+				n = ext[cell];
+				if (mode == 2) {                  // State::likelihood term of the fixed count
+					const double lp = poisson_lp(n, mean);
+					const double t = Lsum + lp;
+					Lcmp += fabs(Lsum) >= fabs(lp) ? (Lsum - t) + lp : (lp - t) + Lsum;
+					Lsum = t;
+				} else {
+					b.ch_mean[chs(cs_p, sett) * tnsz + cell] = mean;
+				}
+				if (copy) tn[cell] = n;
+				continue;
+			}
+			if (!bad && !is_zero(mean)) {
+				if (__double_as_longlong(mean) > __double_as_longlong(1000000000.0)) set_status(status, BEEP_COUNT_OVERFLOW);
 				else {
-					const uint32_t col = (uint32_t)(c * DP + dp);
-					if (mode == 0 || b.simu_all || (b.simu && b.simu[((size_t)p * m.S + sett) * A + c])) {
-						n = poisson_fp64(mean, k0, k1, col, (uint32_t)tr, (uint32_t)sett, stream, lim);
-					} else {                        // coupled to the current state (src/mbp.cc:293-305)
+					// integers equal to the FP64 samplers' (rng_filter.cuh)
+					double draw = mean;
+					int32_t n0 = 0;
+					bool thin = false;
+					double ri = 0.0;
+					if (mode != 0 && !b.simu_all && !(b.simu && b.simu[((size_t)p * m.S + sett) * A + c])) {
+						// coupled to the current state (src/mbp.cc:293-305)
 						const size_t ci = chs(cs_i, sett) * tnsz + cell;
-						const int32_t ni = b.ch_tn[ci];
-						const double ri = b.ch_mean[ci];
-						if (mean > ri) {
-							n = poisson_fp64(mean - ri, k0, k1, col, (uint32_t)tr, (uint32_t)sett, stream, lim);
-							if (n >= 0) n += ni;
-						} else if (mean == ri) n = ni;
-						else n = binomial_fp64(mean / ri, ni, k0, k1, col, (uint32_t)tr, (uint32_t)sett, stream, lim);
+						n0 = b.ch_tn[ci];
+						ri = b.ch_mean[ci];
+						draw = mean - ri;
+						thin = mean < ri;
+					}
+					if (thin) n = binomial_filtered(mean / ri, n0, k0, k1, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, lim, ftab);
+					else {
+						if (draw > 0.0) n = poisson_filtered(draw, k0, k1, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, lim, ftab);
+						if (n >= 0) n += n0;
 					}
 					if (n < 0) { set_status(status, BEEP_TIMEOUT); n = 0; }
 				}
 			}
 			if (mode == 1) b.ch_mean[chs(cs_p, sett) * tnsz + cell] = mean;
 			tn[cell] = n;
+			if (copy) ext[cell] = n;
+		}
+		if (smem_tabs) {
+			double *nb = bea + (buf ^ 1) * NSA, *ne = eta + (buf ^ 1) * NSA, *nn = Nm + (buf ^ 1) * GG;
+			if (tid < NSA) { nb[tid] = nbe; ne[tid] = net; }
+			if (tid < GG) nn[tid] = nN;
+			for (int i = tid + nth; i < NSA; i += nth) slice(sn, i, nb[i], ne[i]);
+			for (int i = tid + nth; i < GG; i += nth) nn[i] = Ntime[(size_t)sn * GG + i];
 		}
 		__syncthreads();
 
 		// ---- E: observation sums (one thread per active observation, cells in reference order)
-		const int s0 = b.step_ptr[sett - b.ti], s1 = mode == 2 ? s0 : b.step_ptr[sett - b.ti + 1];
 		for (int k = s0 + tid; k < s1; k += nth) {
-			const int pos = b.step_obs[k];
-			const int o = b.scored[pos];
-			const double fac = m.obs_factor[o];
-			const int spl = m.obs_spline[o];
-			double v = acc[pos];
-			for (int q = m.obs_cell_ptr[o]; q < m.obs_cell_ptr[o + 1]; q++) {
-				const int cell = m.obs_cells[q];
-				if (cell >= 0) {
-					const double num = (double)tn[cell];
-					if (num != 0) {
-						if (spl < 0) v += fac * num;
-						else v += fac * num * obs_spline[(size_t)spl * m.S + sett];
+			int q0 = oq0, q1 = oq1, spl = ospl, pos = opos;
+			double fac = ofac, v = oacc;
+			if (k != s0 + tid) {
+				pos = b.step_obs[k];
+				const int o = b.scored[pos];
+				q0 = m.obs_cell_ptr[o];
+				q1 = m.obs_cell_ptr[o + 1];
+				spl = m.obs_spline[o];
+				fac = m.obs_factor[o];
+				v = acc[pos];
+			}
+			if (!kPop64 && spl < 0 && __double_as_longlong(fac) == __double_as_longlong(1.0)) {
+				// a unit factor: the counts' sum is an integer, exact in either arithmetic
+				long long sum = 0;
+				for (int q = q0; q < q1; q++) {
+					const int cell = m.obs_cells[q];
+					sum += cell >= 0 ? (long long)tn[cell] : (long long)pop_cur[-1 - cell];
+				}
+				if (sum != 0) v += (double)sum;
+			} else {
+				for (int q = q0; q < q1; q++) {
+					const int cell = m.obs_cells[q];
+					if (cell >= 0) {
+						const double num = (double)tn[cell];
+						if (num != 0) {
+							if (spl < 0) v += fac * num;
+							else v += fac * num * obs_spline[(size_t)spl * m.S + sett];
+						}
+					} else {
+						v += fac * (double)pop_cur[-1 - cell];
 					}
-				} else {
-					v += fac * (double)pop_cur[-1 - cell];
 				}
 			}
 			acc[pos] = v;
 		}
-		// update_pop into the other buffer
-		for (size_t k = tid; k < popsz; k += nth) {
-			const int dp = (int)(k % DP), co = (int)((k / DP) % C), c = (int)(k / ((size_t)DP * C));
+		opos = npos;
+		// update_pop into the other buffer, a column per thread and compartment
+		for (int k = tid; k < (int)popsz; k += nth) {
+			const int cc = divDP.quot(k), dp = k - cc * DP, c = cc / C, co = cc - c * C;
+			const int32_t *tc = tn + (size_t)c * T * DP + dp;
 			if constexpr (kPop64) {
 				// FP64 populations: the flows in transition order, as update_pop applies them
 				double v = pop_cur[k];
 				for (int tr = 0; tr < T; tr++) {
-					const int32_t n = tn[((size_t)c * T + tr) * DP + dp];
+					const int32_t n = tc[tr * DP];
 					if (n != 0) {
-						if (m.trans_from[tr] == co) v -= (double)n;
-						if (m.trans_to[tr] == co) v += (double)n;
+						if (from[tr] == co) v -= (double)n;
+						if (to[tr] == co) v += (double)n;
 					}
 				}
 				pop_nxt[k] = v;
 			} else {
 				long long v = pop_cur[k];
 				for (int tr = 0; tr < T; tr++) {
-					const long long n = tn[((size_t)c * T + tr) * DP + dp];
-					if (m.trans_from[tr] == co) v -= n;
-					if (m.trans_to[tr] == co) v += n;
+					const long long n = tc[tr * DP];
+					if (from[tr] == co) v -= n;
+					if (to[tr] == co) v += n;
 				}
 				if (v > 2147483647ll || v < -2147483648ll) { set_status(status, BEEP_COUNT_OVERFLOW); v = 0; }
 				pop_nxt[k] = (int32_t)v;
 			}
 			if (b.pop_traj) ((PopT *)b.pop_traj)[((size_t)p * nsteps + (sett - b.ti)) * popsz + k] = pop_cur[k];
 		}
+		// ---- A of the next step: dinf from this step's counts (INF_DIF_UPDATE: their differences)
+		if (sett + 1 < b.tf && mode != 2) dinf_of_counts(tn, dif ? b.ch_tn + chs(cs_i, sett) * tnsz : nullptr);
 		__syncthreads();
 		PopT *sw = pop_cur; pop_cur = pop_nxt; pop_nxt = sw;
+		buf ^= 1;
 	}
 
 	if (b.pop_out)
 		for (size_t k = tid; k < popsz; k += nth) ((PopT *)b.pop_out)[(size_t)p * popsz + k] = pop_cur[k];
 
-	__shared__ double part_s[kThreads], part_c[kThreads];
+	__shared__ double part_s[kMaxThreads], part_c[kMaxThreads];
 	if (mode == 2) {
 		// the threads' compensated partial sums, combined in thread order
 		part_s[tid] = Lsum;
@@ -467,12 +628,34 @@ __global__ void __launch_bounds__(kThreads) sim_plain_kernel(const ModelDev m, c
 
 }  // namespace
 
+namespace {
+
+template <typename PopT>
+int launch_pop(const ModelDev &m, const BatchDev &b, cudaStream_t st)
+{
+	// the particle's arrays in shared memory where two CTAs per SM still fit (they leave the
+	// chain of global loads between a step's phases); 512 threads per CTA when each SM holds
+	// one particle anyway and a step has that many draws
+	const size_t most = 104 * 1024;
+	int level = 2;
+	while (level > 0 && PlainSmem(m, (int)sizeof(PopT), level).total > most) level--;
+	const size_t smem = PlainSmem(m, (int)sizeof(PopT), level).total;
+	int dev = 0, sms = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+	if (e == cudaSuccess) e = allow_dynamic_smem(sim_plain_kernel<PopT>, smem);
+	if (e != cudaSuccess) return (int)e;
+	const int nth = b.P <= sms && m.T * m.A * m.DP > 256 ? 512 : 256;
+	sim_plain_kernel<PopT><<<b.P, nth, smem, st>>>(m, b, level);
+	return (int)cudaGetLastError();
+}
+
+}  // namespace
+
 int launch_sim_plain(const ModelDev &m, const BatchDev &b, void *stream)
 {
 	if (b.P == 0) return 0;
-	if (m.ndcc > 0) sim_plain_kernel<double><<<b.P, kThreads, 0, (cudaStream_t)stream>>>(m, b);
-	else sim_plain_kernel<int32_t><<<b.P, kThreads, 0, (cudaStream_t)stream>>>(m, b);
-	return (int)cudaGetLastError();
+	return m.ndcc > 0 ? launch_pop<double>(m, b, (cudaStream_t)stream) : launch_pop<int32_t>(m, b, (cudaStream_t)stream);
 }
 
 }  // namespace beep
