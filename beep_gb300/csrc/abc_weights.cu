@@ -35,8 +35,10 @@
 namespace beep {
 namespace {
 
-constexpr int kAbcThreads = 256;
+constexpr int kAbcThreads = 32;      // new particles per CTA
 constexpr int kAbcTile = 256;        // last-generation particles staged per pass
+constexpr int kAbcGroup = 8;         // terms in flight per thread
+constexpr int kFarThreads = 256;     // threads of the FP64 pass, per new particle
 constexpr int kMaxVar = 16;
 constexpr double kFarExponent = 10.0;
 
@@ -64,47 +66,102 @@ __device__ __forceinline__ R quad_form(const R *d, const R *A, int nvar)
 	return q;
 }
 
-template <bool WHITE>
-__global__ void __launch_bounds__(kAbcThreads) abc_logsums_f32(int nvar, int nnew, const float *z_new, int nlast,
+// Pass 1.  A new particle's terms enter its running log-sum-exp one after another (the
+// running maximum and the compensated sum depend on their order), so a thread owns a new
+// particle and the bound is the latency of its chain of sums: four dependent additions per
+// term.  What feeds the chain is taken off it -- kAbcGroup terms' forms and exponentials are
+// in flight at once, a previous particle (its coordinates and log weight, padded to 16 bytes)
+// loads as one or a few vectors, and only a group that raises the maximum (a handful per
+// particle) or holds a weight of zero goes term by term.  CTAs of one warp put a warp on
+// every scheduler from 608 x 32 new particles.  16384 x 16384, 3 parameters: 3.73 ms as 64
+// CTAs of 256 threads, one term at a time with predicated loops over 16 parameters;
+// 0.56 ms now (71 cycles per term and warp, 29 instructions).
+// NV: the parameters, or 0 for a count only known at run time.
+template <bool WHITE, int NV>
+__global__ void __launch_bounds__(kAbcThreads) abc_logsums_f32(int nvar_, int nnew, const float *z_new, int nlast,
                                                                const float *z_last, const float *logw_last,
                                                                const float *A, double *logsum_out, float *max_out)
 {
-	__shared__ float s_z[kAbcTile * kMaxVar];
-	__shared__ float s_lw[kAbcTile];
+	constexpr int kV = NV > 0 ? NV : kMaxVar, kStride = (kV + 1 + 3) & ~3;
+	__shared__ float4 s_zw[kAbcTile * kStride / 4];      // per previous particle: coordinates, log weight
 	__shared__ float s_A[kMaxVar * kMaxVar];
+	const int nvar = NV > 0 ? NV : nvar_;
 	const int i = blockIdx.x * kAbcThreads + threadIdx.x;
+	float *zw = reinterpret_cast<float *>(s_zw);
 	if (!WHITE)
 		for (int k = threadIdx.x; k < nvar * nvar; k += kAbcThreads) s_A[k] = A[k];
-	float x[kMaxVar];
+	float x[kV];
 #pragma unroll
-	for (int v = 0; v < kMaxVar; v++) x[v] = (i < nnew && v < nvar) ? z_new[(size_t)i * nvar + v] : 0.f;
+	for (int v = 0; v < kV; v++) x[v] = (i < nnew && v < nvar) ? z_new[(size_t)i * nvar + v] : 0.f;
 	float mx = -INFINITY, s = 0.f, cmp = 0.f;      // running max exponent; compensated sum of exp(x_j - mx)
+	auto exponent = [&](int j) {
+		float d[kMaxVar], q4[kStride];
+#pragma unroll
+		for (int k = 0; k < kStride / 4; k++) *reinterpret_cast<float4 *>(q4 + 4 * k) = s_zw[j * (kStride / 4) + k];
+#pragma unroll
+		for (int v = 0; v < kMaxVar; v++) d[v] = v < kV && v < nvar ? x[v < kV ? v : 0] - q4[v < kV ? v : 0] : 0.f;
+		return q4[kV] - 0.5f * quad_form<WHITE>(d, s_A, nvar);
+	};
+	auto add = [&](float term) {
+		const float y = term - cmp;                  // Kahan
+		const float t = s + y;
+		cmp = (t - s) - y;
+		s = t;
+	};
+	auto one = [&](float xe) {
+		if (xe == -INFINITY) return;                 // a previous particle of weight zero
+		if (xe > mx) {                               // new largest exponent: rescale the sum
+			const float f = expf(mx - xe);
+			s *= f;
+			cmp *= f;
+			mx = xe;
+		}
+		add(expf(xe - mx));
+	};
 	for (int j0 = 0; j0 < nlast; j0 += kAbcTile) {
 		const int nj = min(kAbcTile, nlast - j0);
 		__syncthreads();
-		for (int k = threadIdx.x; k < nj * nvar; k += kAbcThreads) s_z[k] = z_last[(size_t)j0 * nvar + k];
-		for (int k = threadIdx.x; k < nj; k += kAbcThreads) s_lw[k] = logw_last[j0 + k];
+		for (int k = threadIdx.x; k < nj * nvar; k += kAbcThreads) zw[k / nvar * kStride + k % nvar] = z_last[(size_t)j0 * nvar + k];
+		for (int k = threadIdx.x; k < nj; k += kAbcThreads) zw[k * kStride + kV] = logw_last[j0 + k];
 		__syncthreads();
-		if (i < nnew) {
-			for (int j = 0; j < nj; j++) {
-				float d[kMaxVar];
+		if (i >= nnew) continue;
+		// the next group's exponents are formed beside this group's chain
+		const int ng = nj / kAbcGroup;
+		float xe[kAbcGroup], xn[kAbcGroup];
+		auto form = [&](float *to, int g) {
 #pragma unroll
-				for (int v = 0; v < kMaxVar; v++) d[v] = v < nvar ? x[v] - s_z[j * nvar + v] : 0.f;
-				const float q = quad_form<WHITE>(d, s_A, nvar);
-				const float xe = s_lw[j] - 0.5f * q;
-				if (xe == -INFINITY) continue;       // a previous particle of weight zero
-				if (xe > mx) {                       // new largest exponent: rescale the sum
-					const float f = expf(mx - xe);
-					s *= f;
-					cmp *= f;
-					mx = xe;
+			for (int u = 0; u < kAbcGroup; u++) to[u] = exponent(g * kAbcGroup + u);
+		};
+		if (ng > 0) form(xn, 0);
+		for (int g = 0; g < ng; g++) {
+			const int gn = min(g + 1, ng - 1);
+			float hi = xn[0], lo = xn[0];
+#pragma unroll
+			for (int u = 0; u < kAbcGroup; u++) {
+				xe[u] = xn[u];
+				hi = fmaxf(hi, xn[u]);
+				lo = fminf(lo, xn[u]);
+			}
+			if (hi <= mx && lo > -INFINITY) {
+				float ex[kAbcGroup];
+#pragma unroll
+				for (int u = 0; u < kAbcGroup; u++) ex[u] = expf(xe[u] - mx);
+				form(xn, gn);
+#pragma unroll
+				for (int u = 0; u < kAbcGroup; u++) add(ex[u]);
+			} else {
+				form(xn, gn);
+#pragma unroll 1
+				for (int u = 0; u < kAbcGroup; u++) {
+					float v = xe[0];
+#pragma unroll
+					for (int w = 1; w < kAbcGroup; w++) v = u == w ? xe[w] : v;
+					one(v);
 				}
-				const float y = expf(xe - mx) - cmp;   // Kahan
-				const float t = s + y;
-				cmp = (t - s) - y;
-				s = t;
 			}
 		}
+		int j = ng * kAbcGroup;
+		for (; j < nj; j++) one(exponent(j));
 	}
 	if (i < nnew) {
 		logsum_out[i] = (double)mx + log((double)s - (double)cmp);
@@ -112,21 +169,22 @@ __global__ void __launch_bounds__(kAbcThreads) abc_logsums_f32(int nvar, int nne
 	}
 }
 
-// FP64 log sums of the listed new particles (one thread each)
+// Pass 2: FP64 log sums of the listed new particles, a CTA each (the FP64 pipe issues one
+// warp instruction per 64 cycles and scheduler: one thread per particle took 26 ms for any
+// number of them at 16384 previous particles)
 template <bool WHITE>
-__global__ void __launch_bounds__(kAbcThreads) abc_logsums_f64(int nvar, int nfar, const int *far_idx,
-                                                               const double *z_new, int nlast, const double *z_last,
+__global__ void __launch_bounds__(kFarThreads) abc_logsums_f64(int nvar, const int *far_idx, const double *z_new,
+                                                               int nlast, const double *z_last,
                                                                const double *logw_last, const double *A,
                                                                double *logsum_out)
 {
-	const int k = blockIdx.x * kAbcThreads + threadIdx.x;
-	if (k >= nfar) return;
-	const int i = far_idx[k];
+	__shared__ double s_m[kFarThreads], s_s[kFarThreads];
+	const int i = far_idx[blockIdx.x], tid = threadIdx.x;
 	double x[kMaxVar];
 #pragma unroll
 	for (int v = 0; v < kMaxVar; v++) x[v] = v < nvar ? z_new[(size_t)i * nvar + v] : 0.0;
 	double mx = -INFINITY, s = 0.0;
-	for (int j = 0; j < nlast; j++) {
+	for (int j = tid; j < nlast; j += kFarThreads) {
 		const double lw = logw_last[j];
 		if (lw == -INFINITY) continue;
 		double d[kMaxVar];
@@ -139,7 +197,39 @@ __global__ void __launch_bounds__(kAbcThreads) abc_logsums_f64(int nvar, int nfa
 		}
 		s += exp(xe - mx);
 	}
-	logsum_out[i] = mx + log(s);
+	s_m[tid] = mx;
+	s_s[tid] = s;
+	for (int o = kFarThreads / 2; o > 0; o >>= 1) {
+		__syncthreads();
+		if (tid >= o) continue;
+		const double m2 = s_m[tid + o], s2 = s_s[tid + o];
+		if (m2 > s_m[tid]) {
+			s_s[tid] = s_s[tid] * exp(s_m[tid] - m2) + s2;
+			s_m[tid] = m2;
+		} else if (m2 > -INFINITY) {
+			s_s[tid] += s2 * exp(m2 - s_m[tid]);
+		} else {
+			s_s[tid] += s2;                            // no term, or NaN
+		}
+	}
+	if (tid == 0) logsum_out[i] = s_m[0] + log(s_s[0]);
+}
+
+using LogSums32 = void (*)(int, int, const float *, int, const float *, const float *, const float *, double *, float *);
+
+template <bool WHITE>
+LogSums32 pick_logsums(int nvar)
+{
+	switch (nvar) {
+	case 1: return abc_logsums_f32<WHITE, 1>;
+	case 2: return abc_logsums_f32<WHITE, 2>;
+	case 3: return abc_logsums_f32<WHITE, 3>;
+	case 4: return abc_logsums_f32<WHITE, 4>;
+	case 5: return abc_logsums_f32<WHITE, 5>;
+	case 6: return abc_logsums_f32<WHITE, 6>;
+	case 7: return abc_logsums_f32<WHITE, 7>;
+	default: return abc_logsums_f32<WHITE, 0>;
+	}
 }
 
 // L with A = L L^T (A symmetric positive definite, row-major n x n); false otherwise
@@ -233,7 +323,7 @@ extern "C" BEEP_API beep_status beep_abcsmc_weights(int32_t nvar, int32_t nnew, 
 	if (e == cudaSuccess) e = cudaMemcpy(d + o_A, Af.data(), 4 * Af.size(), cudaMemcpyHostToDevice);
 	if (e == cudaSuccess) e = cudaMemcpy(d + o_A64, Am.data(), 8 * Am.size(), cudaMemcpyHostToDevice);
 	if (e == cudaSuccess) {
-		auto k32 = white ? abc_logsums_f32<true> : abc_logsums_f32<false>;
+		const LogSums32 k32 = white ? pick_logsums<true>(nvar) : pick_logsums<false>(nvar);
 		k32<<<(nnew + kAbcThreads - 1) / kAbcThreads, kAbcThreads>>>(
 		    nvar, nnew, (const float *)(d + o_zn), nlast, (const float *)(d + o_zl), (const float *)(d + o_wl),
 		    (const float *)(d + o_A), (double *)(d + o_s), (float *)(d + o_mx));
@@ -250,8 +340,8 @@ extern "C" BEEP_API beep_status beep_abcsmc_weights(int32_t nvar, int32_t nnew, 
 			if (e == cudaSuccess) e = cudaMemcpy(d + o_far, far.data(), 4 * far.size(), cudaMemcpyHostToDevice);
 			if (e == cudaSuccess) {
 				auto k64 = white ? abc_logsums_f64<true> : abc_logsums_f64<false>;
-				k64<<<((int)far.size() + kAbcThreads - 1) / kAbcThreads, kAbcThreads>>>(
-				    nvar, (int)far.size(), (const int *)(d + o_far), (const double *)(d + o_zn64), nlast,
+				k64<<<(int)far.size(), kFarThreads>>>(
+				    nvar, (const int *)(d + o_far), (const double *)(d + o_zn64), nlast,
 				    (const double *)(d + o_zl64), (const double *)(d + o_wl64), (const double *)(d + o_A64),
 				    (double *)(d + o_s));
 				e = cudaGetLastError();
