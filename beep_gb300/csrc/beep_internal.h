@@ -71,6 +71,7 @@ struct BatchDev {
 	const uint32_t *stream_of;          // [P] or null
 	const uint2 *key_of;                // [P] Philox key (seed words) of each particle, or null: (k0, k1) for all
 	const int32_t *pop_in;              // [P][A][C][DP] or null (ti == 0)
+	const int32_t *pop_of;              // [P] row of pop_in that each particle starts from, or null: its own
 	// scored observations and their per-step activity
 	int32_t nscored;
 	const int32_t *scored;              // [nscored] ascending obs index

@@ -970,14 +970,8 @@ beep_status beep_batch_upload(beep_batch *q)
 beep_status beep_batch_launch(beep_batch *q)
 {
 	if (!q) return fail(BEEP_BAD_INPUT, "null batch");
-	q->bd.sampler_limit = option_sampler_limit();   // batches kept across calls follow the current option
 	CUDA_TRY(cudaMemsetAsync(q->bd.status, 0, 4 * (size_t)q->bd.P, q->m->stream));
-	int le = q->b.form != BEEP_FORM_FAST ? launch_sim_plain(q->m->dev, q->bd, q->m->stream)
-	         : q->bd.batched              ? launch_sim_batched(q->m->dev, q->bd, q->m->sms, q->m->stream)
-	                                      : launch_sim_fast(q->m->dev, q->bd, q->m->stream);
-	if (le != 0) return fail(BEEP_DEVICE_ERROR, std::string("kernel launch: ") + cudaGetErrorString((cudaError_t)le));
-	q->pending = true;
-	return BEEP_OK;
+	return batch_launch_kernels(q);
 }
 
 beep_status beep_batch_download(beep_batch *q)
@@ -990,6 +984,23 @@ beep_status beep_batch_download(beep_batch *q)
 }
 
 }  // extern "C"
+
+beep_status beep::batch_stage_idle(beep_batch *q)
+{
+	const beep_status st = check_batch(q->m, &q->b, q->device_io);
+	return st != BEEP_OK ? st : stage_inputs(q);
+}
+
+beep_status beep::batch_launch_kernels(beep_batch *q)
+{
+	q->bd.sampler_limit = option_sampler_limit();   // batches kept across calls follow the current option
+	int le = q->b.form != BEEP_FORM_FAST ? launch_sim_plain(q->m->dev, q->bd, q->m->stream)
+	         : q->bd.batched              ? launch_sim_batched(q->m->dev, q->bd, q->m->sms, q->m->stream)
+	                                      : launch_sim_fast(q->m->dev, q->bd, q->m->stream);
+	if (le != 0) return fail(BEEP_DEVICE_ERROR, std::string("kernel launch: ") + cudaGetErrorString((cudaError_t)le));
+	q->pending = true;
+	return BEEP_OK;
+}
 
 beep_status beep::batch_download_enqueue(beep_batch *q)
 {

@@ -158,6 +158,10 @@ namespace beep {
 beep_status batch_create_internal(beep_model *m, const beep_sim_batch *b, bool device_io, beep_batch **out,
                                   bool device_traj = false, bool allow_tc = true, bool allow_ctas = true,
                                   const std::vector<uint2> *keys = nullptr);
+// beep_batch_stage for a caller whose copies from the staging buffer have completed (no wait).
+beep_status batch_stage_idle(beep_batch *q);
+// beep_batch_launch for a caller that has cleared bd.status itself.
+beep_status batch_launch_kernels(beep_batch *q);
 // beep_batch_download in two halves: the device->host copy enqueued on the
 // model's stream, and (once that copy completed) the status check and the
 // copy into the caller's arrays.

@@ -275,9 +275,10 @@ __global__ void __launch_bounds__(256) bx_init(const ModelDev m, const BatchDev 
 	const int p = blockIdx.x, tid = threadIdx.x;
 	const int A = m.A, G = m.G, DP = m.DP, DPS = m.DPS, C = m.C, NS = m.NS, ncol = A * DP, popsz = C * ncol;
 	int32_t *pop = bx_pop(m, b, p, 0);
+	const int src = b.pop_of ? b.pop_of[p] : p;
 	for (int k = tid; k < popsz; k += blockDim.x) {
 		const int dp = k % DP, co = (k / DP) % C, c = k / (DP * C);
-		pop[co * ncol + c * DP + dp] = b.ti == 0 ? m.pop_init[k] : b.pop_in[(size_t)p * popsz + k];
+		pop[co * ncol + c * DP + dp] = b.ti == 0 ? m.pop_init[k] : b.pop_in[(size_t)src * popsz + k];
 	}
 	__syncthreads();
 	if (NS > 1) {

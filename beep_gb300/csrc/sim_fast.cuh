@@ -644,10 +644,11 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 	uint32_t tc_step = 0;
 	if (s.Ms)
 		for (int k = tid; k < A * A; k += NT) s.Ms[(k / A) * lda + k % A] = m.Mdense[k];
+	const int src = b.pop_of ? b.pop_of[p] : p;
 	for (int k = tid; k < popsz; k += NT) {
 		// global layout [c][co][dp] -> shared [co][c*DP+dp]
 		const int dp = k % DP, co = (k / DP) % C, c = k / (DP * C);
-		s.pop0[co * ncol + c * DP + dp] = b.ti == 0 ? m.pop_init[k] : b.pop_in[(size_t)p * popsz + k];
+		s.pop0[co * ncol + c * DP + dp] = b.ti == 0 ? m.pop_init[k] : b.pop_in[(size_t)src * popsz + k];
 	}
 	for (int k = tid; k < b.nslots; k += NT) s.slot[k] = 0.f;
 	for (int k = tid; k < agsz; k += NT) s.Ic1[k] = 0.f;

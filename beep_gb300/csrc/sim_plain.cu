@@ -248,8 +248,9 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 	const bool one_dp = smem_tabs && m.dp_age_unique;
 	int32_t *status = b.status + p;
 
+	const int src = b.pop_of ? b.pop_of[p] : p;
 	for (size_t k = tid; k < popsz; k += nth)
-		pop_cur[k] = b.ti == 0 ? (PopT)m.pop_init[k] : ((const PopT *)b.pop_in)[(size_t)p * popsz + k];
+		pop_cur[k] = b.ti == 0 ? (PopT)m.pop_init[k] : ((const PopT *)b.pop_in)[(size_t)src * popsz + k];
 	for (int k = tid; k < b.nscored; k += nth) acc[k] = 0.0;
 	// tables in shared memory (level >= 1) or where they are
 	auto table = [&](size_t off, const auto *src, int n) {
