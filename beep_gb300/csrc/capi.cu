@@ -8,8 +8,8 @@
 //   2. one host->device copy, the kernel, one device->host copy of the
 //      outputs, all on the model's stream;
 //   3. per-particle status words are reduced to the returned beep_status.
-// Device memory is a per-model arena that only grows, so steady-state calls
-// allocate nothing.
+// Device and pinned memory comes from the model's pool, so calls of the sizes
+// seen before allocate nothing.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -112,6 +112,13 @@ beep_status beep_device_init(int32_t device)
 }
 
 beep_status beep_model_create(const beep_model_desc *d, beep_model **out)
+{
+	return model_create_internal(d, std::make_shared<BufPool>(kModelPoolBytes), out);
+}
+
+}  // extern "C"
+
+beep_status beep::model_create_internal(const beep_model_desc *d, std::shared_ptr<BufPool> pool, beep_model **out)
 {
 	if (!d || !out) return fail(BEEP_BAD_INPUT, "null argument");
 	*out = nullptr;
@@ -308,6 +315,7 @@ beep_status beep_model_create(const beep_model_desc *d, beep_model **out)
 	}
 
 	beep_model *m = new beep_model();
+	m->pool = std::move(pool);
 	m->A = A; m->G = G; m->DP = DP; m->NS = NS; m->C = C; m->T = T; m->S = S;
 	m->period = d->period; m->dpt = d->division_per_time; m->nobs = nobs;
 	m->obs_sett_i.assign(d->obs_sett_i, d->obs_sett_i + nobs);
@@ -368,7 +376,7 @@ beep_status beep_model_create(const beep_model_desc *d, beep_model **out)
 		put(o_df, d->dcc_frac, 8 * (size_t)dcc_nf);
 	}
 	cudaError_t e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
-	if (e == cudaSuccess) e = m->model_mem.reserve(L.size);
+	if (e == cudaSuccess) e = m->model_mem.reserve(L.size, m->pool.get());
 	// on the model's stream, waited for: a cudaMemcpy from pageable memory may return
 	// before its last bytes land, and the model's (non-blocking) stream would not wait for
 	// the legacy stream's copy
@@ -423,6 +431,8 @@ beep_status beep_model_create(const beep_model_desc *d, beep_model **out)
 	return BEEP_OK;
 }
 
+extern "C" {
+
 beep_status beep_model_destroy(beep_model *m)
 {
 	if (!m) return BEEP_OK;
@@ -430,7 +440,7 @@ beep_status beep_model_destroy(beep_model *m)
 	for (beep_batch *q : m->pf.q) beep_batch_destroy(q);
 	m->pf.q.clear();
 	m->pf.work.release();
-	m->model_mem.release();
+	m->model_mem.release(m->pool.get());
 	if (m->stream) cudaStreamDestroy(m->stream);
 	delete m;
 	return BEEP_OK;
@@ -592,8 +602,8 @@ beep_status stage_inputs(beep_batch *q)
 	       o_key = in.add(8 * q->keys.size()),
 	       o_sc = in.add(4 * q->scored.size()), o_sp = in.add(4 * q->step_ptr.size()),
 	       o_sobs = in.add(4 * q->step_obs.size()), o_tasks = in.add(4 * q->tasks.size());
-	CUDA_TRY(q->in_host.reserve(in.size));
-	CUDA_TRY(q->in_dev.reserve(in.size));
+	CUDA_TRY(q->in_host.reserve(in.size, m->pool.get()));
+	CUDA_TRY(q->in_dev.reserve(in.size, m->pool.get()));
 	q->in_size = in.size;
 	char *h = (char *)q->in_host.ptr;
 	memcpy(h + o_dirs, q->dirs.data(), sizeof(GroupDir) * q->dirs.size());
@@ -911,9 +921,9 @@ beep_status beep::batch_create_internal(beep_model *m, const beep_sim_batch *b, 
 	q->u_tn = ou.add(b->transnum_out ? 4 * tnsz * (size_t)nsteps * P : 0);
 	q->u_pt = ou.add(want_pt ? pe * popsz * (size_t)nsteps * P : 0);
 	q->out_size = ou.size;
-	cudaError_t e = q->work_dev.reserve(wk.size);
-	if (e == cudaSuccess) e = q->out_dev.reserve(ou.size);
-	if (e == cudaSuccess) e = q->out_host.reserve(ou.size);
+	cudaError_t e = q->work_dev.reserve(wk.size, m->pool.get());
+	if (e == cudaSuccess) e = q->out_dev.reserve(ou.size, m->pool.get());
+	if (e == cudaSuccess) e = q->out_host.reserve(ou.size, m->pool.get());
 	if (e == cudaSuccess) e = cudaEventCreate(&q->ev0);
 	if (e == cudaSuccess) e = cudaEventCreate(&q->ev1);
 	if (e != cudaSuccess)
@@ -1241,11 +1251,12 @@ beep_status beep_batch_destroy(beep_batch *q)
 {
 	if (!q) return BEEP_OK;
 	if (q->m && q->m->stream) cudaStreamSynchronize(q->m->stream);
-	q->in_host.release();
-	q->out_host.release();
-	q->in_dev.release();
-	q->work_dev.release();
-	q->out_dev.release();
+	BufPool *pool = q->m ? q->m->pool.get() : nullptr;   // (the stream is idle)
+	q->in_host.release(pool);
+	q->out_host.release(pool);
+	q->in_dev.release(pool);
+	q->work_dev.release(pool);
+	q->out_dev.release(pool);
 	if (q->ev0) cudaEventDestroy(q->ev0);
 	if (q->ev1) cudaEventDestroy(q->ev1);
 	for (cudaEvent_t e : q->ev_split) cudaEventDestroy(e);

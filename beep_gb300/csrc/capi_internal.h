@@ -6,6 +6,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -27,49 +28,125 @@ beep_status fail(beep_status s, const std::string &msg);
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// A device buffer that only grows.
-struct DevBuf {
-	void *ptr = nullptr;
-	size_t cap = 0;
-	cudaError_t reserve(size_t n)
+// Device and pinned buffers of destroyed batches and models, kept for the next ones: an
+// allocation, and above all a release, of either kind costs 0.1 to 1 ms and waits for the
+// whole device.  A pool belongs to a model (its batches come and go, one per beep_simulate)
+// or to a server (models and batches per request); it keeps at most `limit` bytes of each kind
+// and goes with its last owner.  Buffers are given back only when no work that uses them is
+// left in flight.  Safe from several threads.
+class BufPool {
+public:
+	explicit BufPool(size_t limit) : limit_(limit) {}
+	~BufPool() { trim(0); }
+	BufPool(const BufPool &) = delete;
+	BufPool &operator=(const BufPool &) = delete;
+	cudaError_t take(bool host, size_t n, void **ptr, size_t *cap)
 	{
-		if (n <= cap) return cudaSuccess;
-		if (ptr) cudaFree(ptr);
-		ptr = nullptr;
-		cap = 0;
-		cudaError_t e = cudaMalloc(&ptr, n);
-		if (e == cudaSuccess) cap = n;
+		// sizes in steps of 1/8 of their power of two, so that batches of near sizes share buffers
+		size_t step = 4096;
+		while (step * 16 < n) step *= 2;
+		n = align_up(n, step);
+		{
+			std::lock_guard<std::mutex> lk(mu_);
+			std::vector<Buf> &v = spare_[host];
+			size_t best = v.size();
+			for (size_t k = 0; k < v.size(); k++)
+				if (v[k].cap >= n && v[k].cap / 4 <= n && (best == v.size() || v[k].cap < v[best].cap)) best = k;
+			if (best < v.size()) {
+				*ptr = v[best].ptr;
+				*cap = v[best].cap;
+				bytes_[host] -= v[best].cap;
+				v.erase(v.begin() + best);
+				return cudaSuccess;
+			}
+		}
+		cudaError_t e = host ? cudaMallocHost(ptr, n) : cudaMalloc(ptr, n);
+		if (e == cudaErrorMemoryAllocation) {
+			cudaGetLastError();
+			trim(0);
+			e = host ? cudaMallocHost(ptr, n) : cudaMalloc(ptr, n);
+		}
+		*cap = e == cudaSuccess ? n : 0;
+		if (e != cudaSuccess) *ptr = nullptr;
 		return e;
 	}
-	void release()
+	void give(bool host, void *ptr, size_t cap)
 	{
-		if (ptr) cudaFree(ptr);
-		ptr = nullptr;
-		cap = 0;
+		{
+			std::lock_guard<std::mutex> lk(mu_);
+			if (bytes_[host] + cap <= limit_ && spare_[host].size() < 256) {
+				spare_[host].push_back(Buf{ptr, cap});
+				bytes_[host] += cap;
+				return;
+			}
+		}
+		drop(host, ptr);
 	}
+	// releases spare buffers, the oldest first, until at most `keep` bytes of each kind are left
+	void trim(size_t keep)
+	{
+		for (int host = 0; host < 2; host++)
+			for (;;) {
+				void *p = nullptr;
+				{
+					std::lock_guard<std::mutex> lk(mu_);
+					if (bytes_[host] <= keep || spare_[host].empty()) break;
+					p = spare_[host].front().ptr;
+					bytes_[host] -= spare_[host].front().cap;
+					spare_[host].erase(spare_[host].begin());
+				}
+				drop(host != 0, p);
+			}
+	}
+	size_t device_bytes()
+	{
+		std::lock_guard<std::mutex> lk(mu_);
+		return bytes_[0];
+	}
+
+private:
+	struct Buf {
+		void *ptr;
+		size_t cap;
+	};
+	static void drop(bool host, void *p)
+	{
+		if (host) cudaFreeHost(p);
+		else cudaFree(p);
+	}
+	std::mutex mu_;
+	std::vector<Buf> spare_[2];          // [0] device, [1] pinned host
+	size_t bytes_[2] = {0, 0}, limit_;
 };
 
-// A pinned host buffer that only grows.
-struct HostBuf {
+// A buffer that only grows, from a pool or from the driver.  (What it held when it grows goes
+// back to the driver, which waits for the work that may still read it.)
+template <bool HOST>
+struct GrowBuf {
 	void *ptr = nullptr;
 	size_t cap = 0;
-	cudaError_t reserve(size_t n)
+	cudaError_t reserve(size_t n, BufPool *pool = nullptr)
 	{
 		if (n <= cap) return cudaSuccess;
-		if (ptr) cudaFreeHost(ptr);
-		ptr = nullptr;
-		cap = 0;
-		cudaError_t e = cudaMallocHost(&ptr, n);
+		release();
+		if (pool) return pool->take(HOST, n, &ptr, &cap);
+		const cudaError_t e = HOST ? cudaMallocHost(&ptr, n) : cudaMalloc(&ptr, n);
 		if (e == cudaSuccess) cap = n;
+		else ptr = nullptr;
 		return e;
 	}
-	void release()
+	void release(BufPool *pool = nullptr)
 	{
-		if (ptr) cudaFreeHost(ptr);
+		if (ptr && pool) pool->give(HOST, ptr, cap);
+		else if (ptr && HOST) cudaFreeHost(ptr);
+		else if (ptr) cudaFree(ptr);
 		ptr = nullptr;
 		cap = 0;
 	}
 };
+using DevBuf = GrowBuf<false>;
+using HostBuf = GrowBuf<true>;
+constexpr size_t kModelPoolBytes = (size_t)256 << 20;   // spare bytes a model keeps, of each kind
 
 // Sequential layout of named regions inside one buffer (256-byte aligned).
 struct Layout {
@@ -96,6 +173,7 @@ struct beep_model {
 	int sms = 152;                // SMs of the device
 	cudaStream_t stream = nullptr;
 	beep::ModelDev dev{};
+	std::shared_ptr<beep::BufPool> pool;   // its batches' buffers
 	beep::DevBuf model_mem;
 	// host copies used to prepare batches
 	int32_t A, G, DP, NS, C, T, S, period, dpt, nobs;
@@ -145,6 +223,8 @@ struct beep_batch {
 
 
 namespace beep {
+// beep_model_create with the model's and its batches' buffers from a pool shared with others.
+beep_status model_create_internal(const beep_model_desc *d, std::shared_ptr<BufPool> pool, beep_model **out);
 // beep_batch_create for internal callers whose start populations and outputs
 // live on the device (device_io: pop_in is not read from the host and the
 // caller sets bd.pop_in / bd.L / bd.pop_out before each launch).

@@ -16,10 +16,11 @@
 //   * creates each admitted request's (or pack's) device model and batch and
 //     enqueues its copies and kernel on the model's own non-blocking stream, so
 //     kernels of different requests run side by side on the SMs they leave free.
-// Device memory of finished requests is released only while nothing runs (or
-// when the oldest request is waiting for that memory): releasing device or
-// pinned memory synchronises the whole device and would stall the kernels of
-// the other requests.
+// Device and pinned memory of finished requests goes to the server's pool, from
+// which later requests take theirs; it is given back to the driver only while
+// nothing runs (down to a model's share) or when the oldest request waits for
+// room: releasing memory synchronises the whole device and would stall the
+// kernels of the other requests.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -153,9 +154,10 @@ struct beep_server {
 	std::mutex mu;
 	std::condition_variable cv_work, cv_done;
 	std::deque<Req *> queue;
-	std::vector<Req *> running, graveyard;
+	std::vector<Req *> running;
+	std::shared_ptr<BufPool> pool;      // the requests' buffers
 	std::map<uint64_t, Req *> reqs;
-	size_t used = 0, held = 0;          // bytes of running requests / of finished ones not yet released
+	size_t used = 0, held = 0;          // bytes of running requests / spare in the pool
 	uint64_t next_id = 1;
 	bool stop = false;
 	std::thread worker;
@@ -167,17 +169,26 @@ struct beep_server {
 
 namespace {
 
-void release_request_memory(Req *r)
-{
-	if (r->pf_thread.joinable()) r->pf_thread.join();
-	if (r->q) beep_batch_destroy(r->q);
-	if (r->m) beep_model_destroy(r->m);
-	if (r->ev_start) cudaEventDestroy(r->ev_start);
-	if (r->ev_end) cudaEventDestroy(r->ev_end);
-	r->q = nullptr;
-	r->m = nullptr;
-	r->ev_start = r->ev_end = nullptr;
-}
+// A request's device objects, taken from it before it is marked done: from then on its
+// record belongs to the caller, who may release it at any time.
+struct ReqObjects {
+	beep_batch *q;
+	beep_model *m;
+	cudaEvent_t ev_start, ev_end;
+	explicit ReqObjects(Req *r) : q(r->q), m(r->m), ev_start(r->ev_start), ev_end(r->ev_end)
+	{
+		r->q = nullptr;
+		r->m = nullptr;
+		r->ev_start = r->ev_end = nullptr;
+	}
+	void destroy()
+	{
+		if (q) beep_batch_destroy(q);
+		if (m) beep_model_destroy(m);
+		if (ev_start) cudaEventDestroy(ev_start);
+		if (ev_end) cudaEventDestroy(ev_end);
+	}
+};
 
 // A particle-filter request runs on its own host thread: the filter steps
 // section by section with host work in between (beep_pf_loglik), so it cannot
@@ -186,7 +197,7 @@ void release_request_memory(Req *r)
 void run_pf_request(beep_server *s, Req *r)
 {
 	cudaSetDevice(s->device);
-	beep_status st = beep_model_create(&r->desc, &r->m);
+	beep_status st = model_create_internal(&r->desc, s->pool, &r->m);
 	if (st == BEEP_OK) {
 		cudaEventCreate(&r->ev_start);
 		cudaEventCreate(&r->ev_end);
@@ -218,7 +229,7 @@ void start_request(beep_server *s, Req *r)
 		r->pf_thread = std::thread(run_pf_request, s, r);
 		return;
 	}
-	beep_status st = beep_model_create(&r->desc, &r->m);
+	beep_status st = model_create_internal(&r->desc, s->pool, &r->m);
 	if (st == BEEP_OK && r->members.size() > 1) {
 		// one batch for the pack: parameter sets, group and stream indices, keys and
 		// start populations of the members one after another
@@ -351,24 +362,23 @@ void worker_main(beep_server *s)
 				x->state = 2;
 			}
 			s->used -= r->bytes;
-			s->held += r->bytes;
-			s->graveyard.push_back(r);
+			ReqObjects objects(r);
 			s->cv_done.notify_all();
-		}
-		// release finished requests' memory while the device is idle, or when
-		// the oldest queued request waits for it
-		const bool head_blocked = !s->queue.empty() && !s->running.empty() &&
-		                          s->used + s->held + s->queue.front()->est > s->budget &&
-		                          s->used + s->queue.front()->est <= s->budget;
-		if (!s->graveyard.empty() && (s->running.empty() || head_blocked)) {
-			std::vector<Req *> g;
-			g.swap(s->graveyard);
-			size_t freed = 0;
-			for (Req *r : g) freed += r->bytes;
-			lk.unlock();
-			for (Req *r : g) release_request_memory(r);
+			lk.unlock();                    // r is the caller's now
+			objects.destroy();
 			lk.lock();
-			s->held -= freed;
+			s->held = s->pool->device_bytes();
+		}
+		// give spare memory back while the device is idle, or when the oldest queued
+		// request waits for it
+		const bool idle = s->running.empty() && s->queue.empty() && s->held > kModelPoolBytes;
+		const bool head_blocked = !s->queue.empty() && s->used + s->held + s->queue.front()->est > s->budget &&
+		                          (s->running.empty() || s->used + s->queue.front()->est <= s->budget);
+		if (s->held > 0 && (idle || head_blocked)) {
+			lk.unlock();
+			s->pool->trim(idle ? kModelPoolBytes : 0);
+			lk.lock();
+			s->held = s->pool->device_bytes();
 		}
 		if (s->stop && s->queue.empty() && s->running.empty()) break;
 		// admit: first fit in arrival order, the oldest request's room held back
@@ -410,9 +420,10 @@ void worker_main(beep_server *s)
 			start_request(s, r);
 			lk.lock();
 			s->used = s->used - r->est + r->bytes;
+			s->held = s->pool->device_bytes();
 			s->running.push_back(r);   // a failed start retires at the next pass
 		}
-		if (s->running.empty() && s->queue.empty() && s->graveyard.empty() && !s->stop) s->cv_work.wait(lk);
+		if (s->running.empty() && s->queue.empty() && !s->stop) s->cv_work.wait(lk);
 		else s->cv_work.wait_for(lk, std::chrono::microseconds(100));
 	}
 }
@@ -438,6 +449,7 @@ BEEP_API beep_status beep_server_create(int32_t device, int64_t hbm_budget_bytes
 	s->device = device;
 	s->budget = (size_t)hbm_budget_bytes;
 	s->max_inflight = max_inflight;
+	s->pool = std::make_shared<BufPool>(s->budget);
 	cudaError_t e = cudaStreamCreateWithFlags(&s->st0, cudaStreamNonBlocking);
 	if (e == cudaSuccess) e = cudaEventCreate(&s->ev0);
 	if (e == cudaSuccess) e = cudaEventRecord(s->ev0, s->st0);
@@ -461,11 +473,7 @@ BEEP_API beep_status beep_server_destroy(beep_server *s)
 	}
 	s->cv_work.notify_all();
 	if (s->worker.joinable()) s->worker.join();
-	for (Req *r : s->graveyard) release_request_memory(r);
-	for (auto &kv : s->reqs) {
-		release_request_memory(kv.second);
-		delete kv.second;
-	}
+	for (auto &kv : s->reqs) delete kv.second;   // (the worker ends after its last request is retired)
 	if (s->ev0) cudaEventDestroy(s->ev0);
 	if (s->st0) cudaStreamDestroy(s->st0);
 	delete s;
@@ -578,8 +586,6 @@ BEEP_API beep_status beep_serve_release(beep_server *s, uint64_t ticket)
 	Req *r = find(s, ticket);
 	if (!r) return fail(BEEP_BAD_INPUT, "unknown ticket");
 	if (r->state != 2) return fail(BEEP_BAD_INPUT, "the request has not finished");
-	if (std::find(s->graveyard.begin(), s->graveyard.end(), r) != s->graveyard.end())
-		return BEEP_OK;   // its memory is released later; the record stays until then
 	s->reqs.erase(ticket);
 	delete r;
 	return BEEP_OK;
