@@ -83,7 +83,7 @@ struct FastSmem {
 	float *dgeo;          // [2] geographic spline value
 	float *red;           // [2*NT]
 	float *mv;            // [T][NT] each thread's transition means (320-thread CTAs, whose registers are tight)
-	float *pm;            // [T][ncol] the step's transition means (draws per (transition, column)), or null
+	int32_t *dn;          // [C][ncol] the step's population changes (draws per (transition, column)), or null
 };
 
 __host__ __device__ inline int ms_lda(int A) { return A + ((40 - A % 32) % 32); }
@@ -405,54 +405,98 @@ struct Tabs {
 // Per-step table slices: beta*areafactor and the external force of infection
 // per (strain, area), the age-mixing matrix and the geographic spline
 // (src/state.cc:403-423, 547-553).  The loads for step sett are issued by
-// slice_load early in the previous step's draw phase (their latency hides
-// behind the draws) and stored by slice_store after it.
+// slice_load early in the previous step's draw phase and stored by slice_store
+// after it.  RAW: what is loaded is combined when it is stored, so that nothing
+// waits for the loads before the draws (small models, whose steps are bound by
+// latency: 1400 cycles of a 7900-cycle step); otherwise it is combined at once,
+// in fewer registers.
 struct SliceRegs {
-	float be, et, N, d;
+	float beta, af, ef, em, N, d;
 };
 
-// item i (strain, area) of a step's slices: beta * areafactor, external force of infection per capita
-__device__ __forceinline__ float2 slice_item(const ModelDev &m, const Tabs &tb, const FastSmem &s, int sett, int i)
+// item i (strain, area) of a step's slices: beta, areafactor, external force of infection and its multiplier
+__device__ __forceinline__ void slice_item(const ModelDev &m, const Tabs &tb, const FastSmem &s, int sett, int i,
+                                           SliceRegs &r)
 {
 	const int A = m.A, c = i % A;
-	const float be = __ldg(tb.beta_rows + (size_t)s.brow[i] * m.S + sett) *
-	                 __ldg(tb.areafactor + (size_t)(sett / m.div_per_time) * A + c);
-	float et = __ldg(tb.efoi_spline + (size_t)s.eref[i] * m.S + sett) * m.inv_popsize_f;
-	if (tb.efoi_mult) et *= __ldg(tb.efoi_mult + ((size_t)sett * A + c) * m.NS + i / A);
-	return make_float2(be, et);
+	r.beta = __ldg(tb.beta_rows + (size_t)s.brow[i] * m.S + sett);
+	r.af = __ldg(tb.areafactor + (size_t)(sett / m.div_per_time) * A + c);
+	r.ef = __ldg(tb.efoi_spline + (size_t)s.eref[i] * m.S + sett);
+	if (tb.efoi_mult) r.em = __ldg(tb.efoi_mult + ((size_t)sett * A + c) * m.NS + i / A);
+}
+
+__device__ __forceinline__ float2 slice_value(const ModelDev &m, const Tabs &tb, const SliceRegs &r)
+{
+	float et = r.ef * m.inv_popsize_f;
+	if (tb.efoi_mult) et *= r.em;
+	return make_float2(r.beta * r.af, et);
 }
 
 // the first NT items of each kind go through registers; items beyond (models
 // with more (strain, area) pairs or age pairs than threads) are loaded when stored
-template <int NT>
+template <int NT, bool RAW = false>
 __device__ __forceinline__ SliceRegs slice_load(const ModelDev &m, const Tabs &tb, const FastSmem &s, int sett, int tid)
 {
-	SliceRegs r{0.f, 0.f, 0.f, 0.f};
+	SliceRegs r{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 	if (tid < m.NS * m.A) {
-		const float2 v = slice_item(m, tb, s, sett, tid);
-		r.be = v.x;
-		r.et = v.y;
+		slice_item(m, tb, s, sett, tid, r);
+		if constexpr (!RAW) {
+			const float2 v = slice_value(m, tb, r);
+			r.beta = v.x;
+			r.ef = v.y;
+		}
 	}
 	if (tid < m.G * m.G) r.N = __ldg(tb.Ntime + (size_t)sett * m.G * m.G + tid);
 	if (tid == 0) r.d = __ldg(tb.geo + sett);
 	return r;
 }
 
-template <int NT>
+template <int NT, bool RAW = false>
 __device__ __forceinline__ void slice_store(const ModelDev &m, const Tabs &tb, FastSmem &s, const SliceRegs &r, int buf,
                                             int sett, int tid)
 {
 	float *be = buf ? s.be1 : s.be0, *et = buf ? s.et1 : s.et0, *N = buf ? s.N1 : s.N0;
 	const int NSA = m.NS * m.A, GG = m.G * m.G;
-	if (tid < NSA) { be[tid] = r.be; et[tid] = r.et; }
+	if (tid < NSA) {
+		const float2 v = RAW ? slice_value(m, tb, r) : make_float2(r.beta, r.ef);
+		be[tid] = v.x;
+		et[tid] = v.y;
+	}
 	if (tid < GG) N[tid] = r.N;
 	if (tid == 0) s.dgeo[buf] = r.d;
 	for (int i = tid + NT; i < NSA; i += NT) {
-		const float2 v = slice_item(m, tb, s, sett, i);
+		SliceRegs q;
+		slice_item(m, tb, s, sett, i, q);
+		const float2 v = slice_value(m, tb, q);
 		be[i] = v.x;
 		et[i] = v.y;
 	}
 	for (int i = tid + NT; i < GG; i += NT) N[i] = __ldg(tb.Ntime + (size_t)sett * GG + i);
+}
+
+// an observation's accumulator v plus its cells of the step, weighted
+__device__ __forceinline__ float obs_add(const ModelDev &m, const BatchDev &b, const Tabs &tb, const int32_t *tn,
+                                         const int32_t *pc, const int4 &t0, const int4 &t1, int sett, float v)
+{
+	const float fac = __int_as_float(t1.x);
+	const int spl = t1.y;
+	const float w = spl < 0 ? fac : fac * tb.obs_spline[(size_t)spl * m.S + sett];
+	const int nc = t0.w & 0x7fffffff;
+	if (t1.w != 0) {                  // consecutive counts or populations: no cell list
+		const int32_t *src = t1.w == 1 ? tn + t0.z : pc + (-1 - t0.z);
+#pragma unroll 4
+		for (int i = 0; i < nc; i++) v = fmaf(w, (float)src[i], v);
+	} else {
+		if (nc > 0) {
+			const int cell = t0.z;
+			v = fmaf(w, cell >= 0 ? (float)tn[cell] : (float)pc[-1 - cell], v);
+		}
+		for (int i = 1; i < nc; i++) {
+			const int cell = __ldg((b.tn_full ? m.obs_cells_full : m.obs_cells_f) + t1.z + i);
+			v = fmaf(w, cell >= 0 ? (float)tn[cell] : (float)pc[-1 - cell], v);
+		}
+	}
+	return v;
 }
 
 // Stirling remainder of log Gamma(z): log Gamma(z) - ((z - 1/2) log z - z + log(2 pi)/2)
@@ -526,6 +570,204 @@ __device__ __forceinline__ int32_t binomial_fp32(float p, int32_t n, uint32_t k0
 // SM grow to 20 / 30 / 40, which hides the latency of the sampler and Philox
 // chains; two of 256 or four of 128 threads for small models.
 constexpr int min_ctas(int nt) { return nt >= 640 ? 1 : nt >= 256 ? 2 : 4; }
+
+// The steps of a small model in a small batch (fast_parallel_draws): the draws of a step one
+// per (transition, column) thread, each with its own mean, so that a step is as long as one
+// draw and not as a column's T draws.  Bound: the latency of a step's dependent phases on one
+// CTA.  Three barriers per step; every global load of a step (tables of the next one, the
+// observation records) is issued before the draws and first used after them; what a thread's
+// draw reads of the model stays in registers over the steps; the counts move populations
+// through an array of changes, so that no copy and no barrier separates means from draws;
+// observations go to the threads after the drawing ones, beside the force of infection.
+// a section of 28 steps for 256 particles of 10 areas x 3 ages: 118 us with the means, the
+// draws and the counts in phases of their own, 88 us now.
+// Returns this thread's place in the reduction of the log-likelihood.
+template <int NT, int MG>
+__device__ __forceinline__ int pd_steps(const ModelDev &m, const BatchDev &b, const Tabs &tb, FastSmem &s, int p,
+                                        uint32_t stream, uint32_t k0, uint32_t k1, int lda, float &Lsum, float &Lcmp,
+                                        bool &cur)
+{
+	constexpr int kItems = 2;                            // (fast_pd_fits)
+	const int tid = threadIdx.x;
+	const int A = m.A, G = m.G, DP = m.DP, NS = m.NS, DPS = m.DPS, C = m.C, T = m.T;
+	const int ncol = A * DP, popsz = C * ncol, tnsz = T * ncol, agsz = NS * A * MG;
+	const int nsteps = b.tf - b.ti, itr = m.infection_trans, inf_from = s.from[itr];
+	const uint32_t lim = b.sampler_limit ? b.sampler_limit : 65536u;
+	const float dt = (float)m.dt;
+	int32_t *status = b.status + p;
+	// this thread's draws; a transition's columns padded to whole warps where the passes stay the same
+	const int pad = (ncol + 31) & ~31, cols = (T * pad + NT - 1) / NT <= (tnsz + NT - 1) / NT ? pad : ncol;
+	const int used = min(NT, (T * cols + 31) & ~31);     // threads that draw in the first pass
+	struct Item {
+		int tr, col, c, a, src, to, row;                 // src, to: its compartments' places in the populations
+		int pool;                                        // the susceptibles it draws on (every strain's: the first's)
+		float rate, sus, fac, dg;
+	} it[kItems];
+#pragma unroll
+	for (int i = 0; i < kItems; i++) {
+		const int idx = tid + i * NT, tr = idx / cols, col = idx - tr * cols;
+		it[i].tr = idx < T * cols && col < ncol ? tr : -1;
+		if (it[i].tr < 0) continue;
+		const int c = col / DP, dp = col - c * DP, st = dp / DPS;
+		it[i].col = col;
+		it[i].c = st * A + c;                            // (strain, area)
+		it[i].a = s.age[dp - st * DPS];
+		it[i].src = s.from[tr] * ncol + col;
+		it[i].to = s.to[tr] * ncol + col;
+		it[i].pool = it[i].src - st * DPS;
+		it[i].row = s.trow[tr];
+		it[i].rate = s.rate[tr * DP + dp];
+		it[i].sus = s.sus[dp];
+		it[i].fac = m.M_factor_f[c];
+		it[i].dg = m.M_diag_f[c];
+	}
+	const int otid = tid >= used ? tid - used : tid + NT - used;   // order of the threads over the observations
+	int sb = 0, a0 = b.step_ptr[0], a1 = b.step_ptr[1];
+	for (int sett = b.ti; sett < b.tf; sett++) {
+		int32_t *pc = cur ? s.pop1 : s.pop0, *pn = cur ? s.pop0 : s.pop1;
+		const SliceRegs nxt = sett + 1 < b.tf ? slice_load<NT, true>(m, tb, s, sett + 1, tid) : SliceRegs{};
+		const int a2 = b.step_ptr[min(sett + 2 - b.ti, nsteps)];
+		int4 t0 = make_int4(0, 0, 0, 0), t1 = make_int4(0, 0, 0, 0);
+		const bool first = a0 + otid < a1;
+		if (first) {
+			t0 = __ldg(b.tasks + 2 * (a0 + otid));
+			t1 = __ldg(b.tasks + 2 * (a0 + otid) + 1);
+		}
+		const float *be = sb ? s.be1 : s.be0, *et = sb ? s.et1 : s.et0, *Nm = sb ? s.N1 : s.N0;
+		const float *Ic_cur = cur ? s.Ic1 : s.Ic0;
+		float *Ic_nxt = cur ? s.Ic0 : s.Ic1;
+		if (NS > 1) {
+			// strain shift of the susceptible population (src/state.cc:392-401)
+			for (int idx = tid; idx < A * DPS; idx += NT) {
+				const int dp = idx % DPS, c = idx / DPS;
+				int32_t *sp = pc + inf_from * ncol + c * DP;
+				int32_t sum = 0;
+				for (int st = 1; st < NS; st++) { sum += sp[DPS * st + dp]; sp[DPS * st + dp] = 0; }
+				sp[dp] += sum;
+			}
+			__syncthreads();
+		}
+		// ---- means and draws
+		const float d = s.dgeo[sb], omd = 1.f - d;
+#pragma unroll
+		for (int i = 0; i < kItems; i++) {
+			const Item &q = it[i];
+			if (q.tr < 0) continue;
+			float mean;
+			if (q.tr == itr) {
+				mean = 0.f;
+				const float popu = (float)pc[q.pool];
+				if (popu > 0.f) {
+					const float fac = q.fac, dg = q.dg;
+					const float *Ic = Ic_cur + q.c * MG, *Im = s.Imap + q.c * MG;
+					const float *N = Nm + q.a * G;
+					float nmi = 0.f;
+#pragma unroll
+					for (int aa = 0; aa < MG; aa++) {
+						if (aa < G) {
+							const float id = Ic[aa] * dg;
+							nmi = fmaf(N[aa], (id + Im[aa]) * d + fac * id * omd, nmi);
+						}
+					}
+					nmi = fmaxf(nmi, 0.f);
+					const float eage = b.nefoi_stage ? s.eage[s.eref[q.c] * G + q.a] : __ldg(tb.efoi_age + (size_t)s.eref[q.c] * G + q.a);
+					mean = dt * popu * q.sus * (be[q.c] * nmi + et[q.c] * eage);
+				}
+			} else {
+				const float popu = (float)pc[q.src];
+				mean = popu <= 0.f ? 0.f : dt * popu * q.rate;
+			}
+			if (tb.tm_mult) mean *= __ldg(tb.tm_mult + ((size_t)sett * A + q.col / DP) * T * DP + q.tr * DP + q.col % DP);
+			U4 inv{0, 0, 0, 0};
+			uint32_t inv_call = 0xffffffffu;
+			int32_t n = 0;
+			if (mean > 0.f) {
+				if (mean > 1.0e9f) atomicCAS(status, 0, BEEP_COUNT_OVERFLOW);
+				else {
+					n = poisson_fp32(mean, k0, k1, (uint32_t)q.col, (uint32_t)q.tr, (uint32_t)sett, stream, inv, inv_call,
+					                 s.rcp, s.lnfact, lim);
+					if (n < 0) { atomicCAS(status, 0, BEEP_TIMEOUT); n = 0; }
+				}
+			} else if (mean != mean) atomicCAS(status, 0, BEEP_NAN_RATE);
+			if (q.row >= 0) s.tn[q.row * ncol + q.col] = n;
+			if (n != 0) {                                // integer changes: their order does not matter
+				atomicSub(s.dn + q.src, n);
+				atomicAdd(s.dn + q.to, n);
+			}
+		}
+		__syncthreads();
+		// ---- populations and infectious counts; the next step's tables
+		int kind = BEEP_OBSVAL_UNKNOWN, model = 0;
+		float2 np = make_float2(0.f, 0.f);
+		float value = 0.f;
+		if (first && t0.w < 0) {                         // an observation to complete: its constants
+			kind = m.obs_kind[t0.y];
+			model = m.obs_model[t0.y];
+			np = m.obs_np[t0.y];
+			value = m.obs_value_f[t0.y];
+		}
+		for (int col = tid; col < ncol; col += NT) {
+			const int c = col / DP, dp = col - c * DP;
+			const int st = dp / DPS, a = s.age[dp - st * DPS];
+			float iv = 0.f;
+			for (int co = 0; co < C; co++) {
+				const int k = co * ncol + col;
+				const int32_t v = pc[k] + s.dn[k];
+				pn[k] = v;
+				s.dn[k] = 0;
+				const float inf = s.inf[co];
+				if (inf != 0.f) iv = fmaf(inf, (float)v, iv);
+			}
+			if (m.dp_age_unique) Ic_nxt[(st * A + c) * MG + a] = iv;
+			else atomicAdd(Ic_nxt + (st * A + c) * MG + a, iv);
+		}
+		if (sett + 1 < b.tf) slice_store<NT, true>(m, tb, s, nxt, sb ^ 1, sett + 1, tid);
+		__syncthreads();
+		// ---- outputs, observations, the next force of infection
+		if (b.pop_traj)
+			for (int k = tid; k < popsz; k += NT) {
+				const int dp = k % DP, co = (k / DP) % C, c = k / (DP * C);
+				b.pop_traj[((size_t)p * nsteps + (sett - b.ti)) * popsz + k] = pc[co * ncol + c * DP + dp];
+			}
+		if (b.tn_traj)
+			for (int k = tid; k < tnsz; k += NT) {
+				const int dp = k % DP, tr = (k / DP) % T, c = k / (DP * T);
+				b.tn_traj[((size_t)p * nsteps + (sett - b.ti)) * tnsz + k] = s.tn[tr * ncol + c * DP + dp];
+			}
+		for (int k = a0 + otid; k < a1; k += NT) {
+			const bool head = k == a0 + otid;
+			if (!head) {
+				t0 = __ldg(b.tasks + 2 * k);
+				t1 = __ldg(b.tasks + 2 * k + 1);
+			}
+			float v = obs_add(m, b, tb, s.tn, pc, t0, t1, sett, s.slot[t0.x]);
+			if (t0.w < 0) {                  // the observation's last step: log-density
+				float lp;
+				if (head && kind == BEEP_OBSVAL_VALUE && (model == BEEP_OBS_NORMAL || model == BEEP_OBS_NORMAL_PERCENT)) {
+					const float dv = value - (v < 0.f ? 0.f : v);
+					lp = np.x - dv * dv * np.y;
+				} else {
+					lp = obs_lp_fast(v, t0.y, m);
+				}
+				v = 0.f;
+				const float y = lp - Lcmp;      // Kahan
+				const float tt = Lsum + y;
+				Lcmp = (tt - Lsum) - y;
+				Lsum = tt;
+			}
+			s.slot[t0.x] = v;
+		}
+		if (!m.dp_age_unique)
+			for (int k = tid; k < agsz; k += NT) (cur ? s.Ic1 : s.Ic0)[k] = 0.f;   // next step's accumulation target
+		foi<NT, MG>(m, s.Ms, lda, Ic_nxt, s.Imap, tid);
+		__syncthreads();
+		cur = !cur;
+		sb ^= 1;
+		a0 = a1;
+		a1 = a2;
+	}
+	return otid;
+}
 
 // One particle (or MBP chain) p of a batch over its whole step range, run by
 // the NT threads of a CTA.  MT: the most transitions the per-column mean
@@ -608,7 +850,7 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 		s.dgeo = (float *)take(4 * 2);
 		s.red = (float *)take(4 * 2 * (size_t)NT);
 		s.mv = NT == kDualThreads ? (float *)take(4 * (size_t)T * NT) : nullptr;
-		s.pm = PD ? (float *)take(4 * (size_t)T * ncol) : nullptr;
+		s.dn = PD ? (int32_t *)take(4 * (size_t)C * ncol) : nullptr;
 	}
 	// tensor-core FOI (large models, 640 threads): chunk ring, stacked counts, barriers, tensor memory
 	__shared__ uint64_t tc_bars[2 * tc::kStages + 1];
@@ -651,6 +893,7 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 		s.pop0[co * ncol + c * DP + dp] = b.ti == 0 ? m.pop_init[k] : b.pop_in[(size_t)src * popsz + k];
 	}
 	for (int k = tid; k < b.nslots; k += NT) s.slot[k] = 0.f;
+	for (int k = tid; PD && k < popsz; k += NT) s.dn[k] = 0;
 	for (int k = tid; k < agsz; k += NT) s.Ic1[k] = 0.f;
 	for (int k = tid; k < T; k += NT) {
 		s.from[k] = m.trans_from[k];
@@ -697,9 +940,11 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 	const float dt = (float)m.dt;
 	bool cur = false;
 	int sb = 0;                                          // slice buffer of the step simulated
-	for (int sett = b.ti; sett < b.tf && tc_ok; sett++) {
+	int red_at = tid;                                    // where this thread's log-likelihood enters the reduction
+	if constexpr (PD) red_at = pd_steps<NT, MG>(m, b, tb, s, p, stream, k0, k1, lda, Lsum, Lcmp, cur);
+	for (int sett = b.ti; sett < b.tf && tc_ok && !PD; sett++) {
 		int32_t *pc = cur ? s.pop1 : s.pop0, *pn = cur ? s.pop0 : s.pop1;
-		const SliceRegs nxt = sett + 1 < b.tf ? slice_load<NT>(m, tb, s, sett + 1, tid) : SliceRegs{0.f, 0.f, 0.f, 0.f};
+		const SliceRegs nxt = sett + 1 < b.tf ? slice_load<NT>(m, tb, s, sett + 1, tid) : SliceRegs{};
 		const float *be = sb ? s.be1 : s.be0, *et = sb ? s.et1 : s.et0, *Nm = sb ? s.N1 : s.N0;
 		const float *Ic_cur = cur ? s.Ic1 : s.Ic0;
 		float *Ic_nxt = cur ? s.Ic0 : s.Ic1;
@@ -717,82 +962,6 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 
 		// ---- A: per column (c, dp): NMI, means, draws, next population and infectious count
 		const float d = s.dgeo[sb], omd = 1.f - d;
-		if constexpr (PD) {
-		// ---- A, small models: the means of every column, then one draw per (transition,
-		//      column) -- the draws of a column run on T threads at once instead of one after
-		//      another on one -- then every column's next infectious count
-		for (int col = tid; col < ncol; col += NT) {
-			const int c = col / DP, dp = col - c * DP;
-			const int st = dp / DPS, dpl = dp - st * DPS, a = s.age[dpl];
-			float minf = 0.f;
-			{
-				const float popu = (float)pc[inf_from * ncol + c * DP + dpl];
-				if (popu > 0.f) {
-					const float fac = m.M_factor_f[c], dg = m.M_diag_f[c];
-					const float *Ic = Ic_cur + (st * A + c) * MG, *Im = s.Imap + (st * A + c) * MG;
-					const float *N = Nm + a * G;
-					float nmi = 0.f;
-#pragma unroll
-					for (int aa = 0; aa < MG; aa++) {
-						if (aa < G) {
-							const float id = Ic[aa] * dg;
-							nmi = fmaf(N[aa], (id + Im[aa]) * d + fac * id * omd, nmi);
-						}
-					}
-					nmi = fmaxf(nmi, 0.f);
-					const int sc = st * A + c;
-					const float eage = b.nefoi_stage ? s.eage[s.eref[sc] * G + a] : __ldg(tb.efoi_age + (size_t)s.eref[sc] * G + a);
-					minf = dt * popu * s.sus[dp] * (be[sc] * nmi + et[sc] * eage);
-				}
-			}
-			for (int tr = 0; tr < T; tr++) {
-				float v;
-				if (tr == itr) v = minf;
-				else {
-					const float popu = (float)pc[s.from[tr] * ncol + col];
-					v = popu <= 0.f ? 0.f : dt * popu * s.rate[tr * DP + dp];
-				}
-				if (tb.tm_mult) v *= __ldg(tb.tm_mult + ((size_t)sett * A + c) * T * DP + tr * DP + dp);
-				s.pm[tr * ncol + col] = v;
-			}
-			if (pn != pc)
-				for (int co = 0; co < C; co++) pn[co * ncol + col] = pc[co * ncol + col];
-		}
-		__syncthreads();
-		for (int idx = tid; idx < T * ncol; idx += NT) {
-			const int tr = idx / ncol, col = idx - tr * ncol;
-			const float mean = s.pm[idx];
-			U4 inv{0, 0, 0, 0};
-			uint32_t inv_call = 0xffffffffu;
-			int32_t n = 0;
-			if (mean > 0.f) {
-				if (mean > 1.0e9f) atomicCAS(status, 0, BEEP_COUNT_OVERFLOW);
-				else {
-					n = poisson_fp32(mean, k0, k1, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, inv, inv_call,
-					                 s.rcp, s.lnfact, lim);
-					if (n < 0) { atomicCAS(status, 0, BEEP_TIMEOUT); n = 0; }
-				}
-			} else if (mean != mean) atomicCAS(status, 0, BEEP_NAN_RATE);
-			const int row = s.trow[tr];
-			if (row >= 0) s.tn[row * ncol + col] = n;
-			if (n != 0) {                                // integer updates: their order does not matter
-				atomicSub(pn + s.from[tr] * ncol + col, n);
-				atomicAdd(pn + s.to[tr] * ncol + col, n);
-			}
-		}
-		__syncthreads();
-		for (int col = tid; col < ncol; col += NT) {
-			const int c = col / DP, dp = col - c * DP;
-			const int st = dp / DPS, dpl = dp - st * DPS, a = s.age[dpl];
-			float iv = 0.f;
-			for (int co = 0; co < C; co++) {
-				const float inf = s.inf[co];
-				if (inf != 0.f) iv = fmaf(inf, (float)pn[co * ncol + col], iv);
-			}
-			if (m.dp_age_unique) Ic_nxt[(st * A + c) * MG + a] = iv;
-			else atomicAdd(Ic_nxt + (st * A + c) * MG + a, iv);
-		}
-		} else {
 		for (int col = tid; col < ncol; col += NT) {
 			const int c = col / DP, dp = col - c * DP;
 			const int st = dp / DPS, dpl = dp - st * DPS, a = s.age[dpl];
@@ -917,7 +1086,6 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 			if (m.dp_age_unique) Ic_nxt[(st * A + c) * MG + a] = iv;
 			else atomicAdd(Ic_nxt + (st * A + c) * MG + a, iv);
 		}
-		}
 		if (sett + 1 < b.tf) slice_store<NT>(m, tb, s, nxt, sb ^ 1, sett + 1, tid);
 		__syncthreads();
 
@@ -940,25 +1108,7 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 		const int a0 = b.step_ptr[sett - b.ti], a1 = b.step_ptr[sett - b.ti + 1];
 		for (int k = a0 + tid - ow; tid >= ow && k < a1; k += NT - ow) {
 			const int4 t0 = __ldg(b.tasks + 2 * k), t1 = __ldg(b.tasks + 2 * k + 1);
-			const float fac = __int_as_float(t1.x);
-			const int spl = t1.y;
-			const float w = spl < 0 ? fac : fac * tb.obs_spline[(size_t)spl * m.S + sett];
-			const int nc = t0.w & 0x7fffffff;
-			float v = s.slot[t0.x];
-			if (t1.w != 0) {                  // consecutive counts or populations: no cell list
-				const int32_t *src = t1.w == 1 ? s.tn + t0.z : pc + (-1 - t0.z);
-#pragma unroll 4
-				for (int i = 0; i < nc; i++) v = fmaf(w, (float)src[i], v);
-			} else {
-				if (nc > 0) {
-					const int cell = t0.z;
-					v = fmaf(w, cell >= 0 ? (float)s.tn[cell] : (float)pc[-1 - cell], v);
-				}
-				for (int i = 1; i < nc; i++) {
-					const int cell = __ldg((b.tn_full ? m.obs_cells_full : m.obs_cells_f) + t1.z + i);
-					v = fmaf(w, cell >= 0 ? (float)s.tn[cell] : (float)pc[-1 - cell], v);
-				}
-			}
+			float v = obs_add(m, b, tb, s.tn, pc, t0, t1, sett, s.slot[t0.x]);
 			if (t0.w < 0) {                  // the observation's last step: log-density
 				const float lp = obs_lp_fast(v, t0.y, m);
 				v = 0.f;
@@ -1017,8 +1167,8 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 	}
 	if (b.L) {
 		__syncthreads();
-		s.red[tid] = Lsum;
-		s.red[NT + tid] = Lcmp;
+		s.red[red_at] = Lsum;
+		s.red[NT + red_at] = Lcmp;
 		__syncthreads();
 		if (tid < 32) {
 			double S = 0.0;
