@@ -110,6 +110,7 @@ struct BatchDev {
 	double *ch_mean;                    // [2][P][S][A][T][DP]
 	double *ch_Imap, *ch_Idiag;         // [2][P][S][NS][A][G]
 	double *Li;                         // [P] mode 2 output
+	int32_t ch_queue;                   // fast form chains: proposals queue their draws (set by the launchers)
 	float *ch_mean_f;                   // fast form chains: means [2][P][S][T][A*DP] (counts in ch_tn, same layout)
 	// fast form: force of infection on the tensor cores (foi_tc.cuh); its shared
 	// memory starts at tc_smem_off bytes into the dynamic shared memory

@@ -29,12 +29,18 @@ int launch_chain_nt(const ModelDev &m, const BatchDev &b, size_t smem, cudaStrea
 
 }  // namespace
 
-int launch_sim_fast_chain(const ModelDev &m, const BatchDev &b, void *stream)
+int launch_sim_fast_chain(const ModelDev &m, const BatchDev &b_, void *stream)
 {
-	if (m.G > 16 || m.T > kMaxT || b.foi_tc || !b.ch_tn || !b.ch_mean_f) return (int)cudaErrorInvalidValue;
-	const int nt = b.nt > 0 ? b.nt : fast_pick_threads(m);
-	const size_t smem = fast_smem_bytes(m, b.nslots, b.m_in_smem != 0, b.nefoi_stage, b.gstate != nullptr,
-	                                    b.tn_full ? m.T : m.tn_rows, b.pop_single != 0, b.tn_smem != 0, nt);
+	if (m.G > 16 || m.T > kMaxT || b_.foi_tc || !b_.ch_tn || !b_.ch_mean_f) return (int)cudaErrorInvalidValue;
+	const int nt = b_.nt > 0 ? b_.nt : fast_pick_threads(m);
+	size_t smem = fast_smem_bytes(m, b_.nslots, b_.m_in_smem != 0, b_.nefoi_stage, b_.gstate != nullptr,
+	                              b_.tn_full ? m.T : m.tn_rows, b_.pop_single != 0, b_.tn_smem != 0, nt);
+	// a proposal's draws are queued where the queue fits beside the chain's state (all of an
+	// SM's chains)
+	BatchDev b = b_;
+	const size_t queue = chain_queue_bytes(m.T, m.C, nt), share = kSmemPerSM / (nt == kDualThreads ? b.ctas : 1) - 1024;
+	b.ch_queue = b.mode == 1 && !b.simu_all && smem + queue <= share && smem + queue <= 227 * 1024 ? 1 : 0;
+	if (b.ch_queue) smem += queue;
 	if (nt == kDualThreads) return launch_sim_fast_chain_ctas(m, b, smem, stream);
 	if (nt != fast_pick_threads(m)) return (int)cudaErrorInvalidValue;
 	const int e = prepare_constants();

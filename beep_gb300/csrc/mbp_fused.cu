@@ -82,7 +82,10 @@ int launch_sim_fast_chain_fused(const ModelDev *m, const BatchDev *b, int n, int
 		f.m[k] = m[k];
 		f.b[k] = b[k];
 		f.first[k + 1] = f.first[k] + b[k].P;
-		smem = std::max(smem, fused_smem_bytes(m[k], b[k], mg));
+		// the set's draws are queued where the queue fits beside its chains' state
+		const size_t need = fused_smem_bytes(m[k], b[k], mg), queue = chain_queue_bytes(m[k].T, m[k].C, kFusedThreads);
+		f.b[k].ch_queue = need + queue <= 226 * 1024 ? 1 : 0;
+		smem = std::max(smem, need + (f.b[k].ch_queue ? queue : 0));
 	}
 	f.nitem = f.first[n];
 	if (f.nitem == 0) return 0;

@@ -84,6 +84,7 @@ struct FastSmem {
 	float *red;           // [2*NT]
 	float *mv;            // [T][NT] each thread's transition means (320-thread CTAs, whose registers are tight)
 	int32_t *dn;          // [C][ncol] the step's population changes (draws per (transition, column)), or null
+	unsigned char *queue; // each warp's queued draws (MBP chains, chain_queue_bytes), or null
 };
 
 __host__ __device__ inline int ms_lda(int A) { return A + ((40 - A % 32) % 32); }
@@ -220,6 +221,11 @@ __device__ float obs_lp_fast(float vf, int o, const ModelDev &m)
 //    of matrix entries loads as one float2, eight sources in flight per lane
 //    (four in the 320-thread layouts).
 // The quad's partial sums are combined with two butterfly shuffles.
+// From 128 areas four targets per quad instead of two (640 threads, up to 12 ages: beyond, the
+// sums do not fit the registers): half the shared-memory reads per product, which bound the
+// other form (350 areas x 10 ages: 80,000 cycles per step before, 48,000 now).
+constexpr int kFoi4Areas = 128;
+
 template <int NT, int MG>
 __device__ __forceinline__ void foi(const ModelDev &m, const float *Ms, int lda, const float *Icnt, float *Imap, int tid)
 {
@@ -258,6 +264,78 @@ __device__ __forceinline__ void foi(const ModelDev &m, const float *Ms, int lda,
 					float4 *Yt = reinterpret_cast<float4 *>(Y + t * MG);
 #pragma unroll
 					for (int q = 0; q < MG / 4; q++) Yt[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+				}
+			}
+		} else if (NT >= 640 && MG <= 12 && A >= kFoi4Areas) {
+			// four targets per quad: a source's counts, read from shared memory, serve twice the
+			// products, and the next four sources' entries are in flight while these are used
+			constexpr int kU = 4;
+			const int nq = (A + 3) / 4;
+			for (int q0 = 0; q0 < nq; q0 += NT / 4) {
+				const int t = 4 * (q0 + (tid >> 2));
+				if (q0 + ((tid & ~31) >> 2) >= nq) break;        // (whole warps)
+				float acc[4][MG];
+#pragma unroll
+				for (int j = 0; j < 4; j++)
+#pragma unroll
+					for (int a = 0; a < MG; a++) acc[j][a] = 0.f;
+				float4 mv[kU], mn[kU];
+				auto load = [&](float4 *to, int cb) {
+#pragma unroll
+					for (int u = 0; u < kU; u++) {
+						const int c = cb + 4 * u;
+						to[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+						if (c < A && t < A) {
+							const float *row = m.Mdense + (size_t)c * A + t;
+							if ((A & 3) == 0) to[u] = __ldg(reinterpret_cast<const float4 *>(row));
+							else if ((A & 1) == 0) {
+								const float2 x = __ldg(reinterpret_cast<const float2 *>(row));
+								const float2 y = t + 2 < A ? __ldg(reinterpret_cast<const float2 *>(row + 2)) : make_float2(0.f, 0.f);
+								to[u] = make_float4(x.x, x.y, y.x, y.y);
+							} else {
+								to[u] = make_float4(__ldg(row), t + 1 < A ? __ldg(row + 1) : 0.f, t + 2 < A ? __ldg(row + 2) : 0.f,
+								                    t + 3 < A ? __ldg(row + 3) : 0.f);
+							}
+						}
+					}
+				};
+				load(mn, cg);
+				for (int cb = cg; cb < A; cb += 4 * kU) {
+#pragma unroll
+					for (int u = 0; u < kU; u++) mv[u] = mn[u];
+					load(mn, cb + 4 * kU);
+#pragma unroll
+					for (int u = 0; u < kU; u++) {
+						const int c = cb + 4 * u;
+						if (c < A) {
+							const float4 *Ic = reinterpret_cast<const float4 *>(I + c * MG);
+							const float w[4] = {mv[u].x, mv[u].y, mv[u].z, mv[u].w};
+#pragma unroll
+							for (int q = 0; q < MG / 4; q++) {
+								const float4 v = Ic[q];
+#pragma unroll
+								for (int j = 0; j < 4; j++) {
+									acc[j][4 * q] = fmaf(w[j], v.x, acc[j][4 * q]);
+									acc[j][4 * q + 1] = fmaf(w[j], v.y, acc[j][4 * q + 1]);
+									acc[j][4 * q + 2] = fmaf(w[j], v.z, acc[j][4 * q + 2]);
+									acc[j][4 * q + 3] = fmaf(w[j], v.w, acc[j][4 * q + 3]);
+								}
+							}
+						}
+					}
+				}
+#pragma unroll
+				for (int j = 0; j < 4; j++) {
+#pragma unroll
+					for (int a = 0; a < MG; a++) {
+						acc[j][a] += __shfl_xor_sync(0xffffffffu, acc[j][a], 1);
+						acc[j][a] += __shfl_xor_sync(0xffffffffu, acc[j][a], 2);
+					}
+					if (t + j < A && cg == j) {                    // (each lane of the quad writes one target)
+						float4 *Yt = reinterpret_cast<float4 *>(Y + (t + j) * MG);
+#pragma unroll
+						for (int q = 0; q < MG / 4; q++) Yt[q] = make_float4(acc[j][4 * q], acc[j][4 * q + 1], acc[j][4 * q + 2], acc[j][4 * q + 3]);
+					}
 				}
 			}
 		} else {
@@ -564,6 +642,303 @@ __device__ __forceinline__ int32_t binomial_fp32(float p, int32_t n, uint32_t k0
 	return flip ? n - k : k;
 }
 
+// ---- Draws of MBP proposals, queued by kind -------------------------------------
+//
+// A coupled cell draws from one of four samplers (Poisson or binomial, by inversion or by
+// rejection), and a column's six cells rarely agree; and each cell's current count and mean
+// come from HBM.  Drawn where they stand, a warp paid for all four samplers in every transition
+// and for each transition's loads in turn.  Here a warp copies the current state of its next
+// 32 columns to shared memory while it draws these, forms the means of their T cells, settles
+// the ones without a draw and queues the others in four lists, which it works through 32 at a
+// time; then it applies the counts to the populations, kept in shared memory meanwhile.  Draws
+// are keyed by (column, step, transition), so their order does not matter: the counts are those
+// of poisson_fp32 and binomial_fp32.  Used where the queue fits beside the chain's state
+// (128 chains each of 20x2, 80x4, 200x6, 350x10 over 400 steps: 69.1 ms per sweep before,
+// 61.9 ms with it and the four-target force of infection; the lists alone gave nothing).
+// Bound: SM issue at five warps per scheduler (57% of the slots), then the matrix's way from L2.
+
+// bytes of one warp: T x 32 of {staged current count, staged current mean, parameter, count, two list
+// entries}, C x 32 populations
+__host__ __device__ inline size_t chain_queue_row(int T, int C) { return (size_t)T * 32 * 18 + (size_t)C * 128; }
+__host__ __device__ inline size_t chain_queue_bytes(int T, int C, int nt) { return (size_t)(nt / 32) * chain_queue_row(T, C); }
+
+__device__ __forceinline__ void copy_async4(void *smem, const void *gmem)
+{
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+
+struct DrawKey {
+	uint32_t k0, k1, sett, stream, lim;
+};
+
+// poisson_fp32 in parts (its words and arithmetic): inversion, and a PTRS trial as a quick
+// decision and a density test
+__device__ __forceinline__ int32_t poisson_inversion(float mean, uint32_t col, uint32_t tr, const DrawKey &q, const float *rcp)
+{
+	const U4 r = philox10(U4{col, q.sett, q.stream, (PURPOSE_INV << 24) | (tr >> 2)}, q.k0, q.k1);
+	const float u = u01_f(word_of(r, tr & 3u));
+	float p = expf(-mean), F = p;
+	int32_t k = 0;
+	while (u > F && k < 63) {
+		k++;
+		p = p * mean * rcp[k];
+		const float Fn = F + p;
+		if (Fn == F) break;
+		F = Fn;
+	}
+	return k;
+}
+
+enum { kPtrsYes, kPtrsNo, kPtrsTest };
+
+__device__ __forceinline__ int ptrs_quick(float mean, float U, float V, float us, float &k)
+{
+	const float slam = sqrtf(mean);
+	const float b = 0.931f + 2.53f * slam;
+	const float a = -0.059f + 0.02483f * b;
+	const float vr = 0.9277f - __fdividef(3.6224f, b - 2.0f);
+	const float two_a = 2.0f * a;
+	k = floorf((__fdividef(two_a, us) + b) * U + mean + 0.43f);
+	if (us >= 0.07f && V <= vr) return kPtrsYes;
+	return k < 0.0f || (us < 0.013f && V > us) ? kPtrsNo : kPtrsTest;
+}
+
+__device__ __forceinline__ bool ptrs_test(float mean, float V, float us, float k, const float *lnfact)
+{
+	const float slam = sqrtf(mean);
+	const float b = 0.931f + 2.53f * slam;
+	const float a = -0.059f + 0.02483f * b;
+	const float loglam = __logf(mean);
+	const float invalpha = 1.1239f + __fdividef(1.1328f, b - 3.4f);
+	float log_invalpha = __logf(invalpha);
+	// rounded before the sum, as in poisson_fp32, which forms it ahead of the trials: fused into
+	// the sum it would decide one draw in 3e8 otherwise
+	asm("mov.f32 %0, %0;" : "+f"(log_invalpha));
+	const float lhs = __logf(V) + log_invalpha - __logf(__fdividef(a, us * us) + b);
+	return lhs <= ptrs_rhs(k, mean, loglam, lnfact);
+}
+
+// PTRS draws of a list: a trial per lane and round; a lane whose draw is settled takes the
+// next one, and the density test, which one trial in six needs, waits until 12 lanes need it.
+// add(id, k): the draw's count, -1 after q.lim rejections.
+template <typename At, typename Add>
+__device__ __forceinline__ void ptrs_list(int n, const float *mean, uint32_t col0, const DrawKey &q, const float *lnfact,
+                                          int lane, At at, Add add)
+{
+	constexpr unsigned kAll = 0xffffffffu;
+	const unsigned below = (1u << lane) - 1u;
+	int id = lane < n ? at(lane) : -1, head = 32;
+	uint32_t it = 0;
+	bool test = false;                                   // this lane's trial waits for the density test
+	float k = 0.f, us = 0.f, V = 0.f;
+	for (;;) {
+		int verdict = kPtrsTest;
+		if (id >= 0 && !test) {
+			const U4 r = philox10(U4{col0 + (uint32_t)(id & 31), q.sett, q.stream,
+			                         (PURPOSE_PTRS << 24) | ((uint32_t)(id >> 5) << 16) | it}, q.k0, q.k1);
+			const float U = u01_f(r.x) - 0.5f;
+			V = u01_f(r.y);
+			us = 0.5f - fabsf(U);
+			verdict = ptrs_quick(mean[id], U, V, us, k);
+			test = verdict == kPtrsTest;
+		}
+		const unsigned waiting = __ballot_sync(kAll, test);
+		if (__popc(waiting) >= 12 ||
+		    (head >= n && !__any_sync(kAll, id >= 0 && !test && verdict != kPtrsYes))) {   // no other lane to try on
+			if (test) verdict = ptrs_test(mean[id], V, us, k, lnfact) ? kPtrsYes : kPtrsNo;
+			test = false;
+		}
+		if (verdict == kPtrsNo && ++it >= q.lim) {
+			k = -1.f;
+			verdict = kPtrsYes;
+		}
+		if (verdict == kPtrsYes && id >= 0) {
+			add(id, (int32_t)k);
+			id = -1;
+		}
+		const unsigned done = __ballot_sync(kAll, id < 0);
+		if (head < n) {
+			const int h = head + __popc(done & below);
+			if (id < 0 && h < n) {
+				id = at(h);
+				it = 0;
+			}
+			head += __popc(done);
+		} else if (done == kAll) break;
+	}
+}
+
+// A proposal's columns (c, dp) of one step: means, coupled draws (src/mbp.cc:293-305), the
+// chain's arrays, populations and next infectious counts.
+template <int NT, int MG>
+__device__ __forceinline__ void chain_columns(const ModelDev &m, const BatchDev &b, const Tabs &tb, const FastSmem &s,
+                                              int p, int sett, const DrawKey &q, const int32_t *pc, int32_t *pn,
+                                              const float *Ic_cur, float *Ic_nxt, const float *be, const float *et,
+                                              const float *Nm, float d, float omd, int cs_i, int cs_p)
+{
+	constexpr unsigned kAll = 0xffffffffu;
+	const int tid = threadIdx.x, lane = tid & 31;
+	const int A = m.A, G = m.G, DP = m.DP, DPS = m.DPS, C = m.C, T = m.T, ncol = A * DP, itr = m.infection_trans;
+	const int inf_from = s.from[itr];
+	const float dt = (float)m.dt;
+	const unsigned below = (1u << lane) - 1u;
+	int32_t *status = b.status + p;
+	// this warp's queue: per cell (transition * 32 + lane) the current state's count and mean, the
+	// draw's parameter and its count so far, the column's populations, and two lists filled from
+	// both ends
+	unsigned char *qw = s.queue + (size_t)(tid >> 5) * chain_queue_row(T, C);
+	int32_t *cur_n = (int32_t *)qw;
+	float *cur_m = (float *)(qw + (size_t)T * 128);
+	float *par = (float *)(qw + (size_t)T * 256);
+	int32_t *cnt = (int32_t *)(qw + (size_t)T * 384);
+	int32_t *pv = (int32_t *)(qw + (size_t)T * 512) + lane;
+	uint8_t *lp = qw + (size_t)T * 512 + (size_t)C * 128, *lb = lp + T * 32;
+	const int last = T * 32 - 1;
+	const size_t cells = (size_t)T * ncol;
+	const int32_t *tn_i = b.ch_tn + (((size_t)cs_i * b.P + p) * m.S + sett) * cells;
+	const float *mean_i = b.ch_mean_f + (((size_t)cs_i * b.P + p) * m.S + sett) * cells;
+	int32_t *tn_p = b.ch_tn + (((size_t)cs_p * b.P + p) * m.S + sett) * cells;
+	float *mean_p = b.ch_mean_f + (((size_t)cs_p * b.P + p) * m.S + sett) * cells;
+	// the current state's cells of a group of columns, copied while the group before is drawn
+	// (they are not written during the proposal)
+	auto stage = [&](int col0) {
+		const int cl = min(col0 + lane, ncol - 1);
+		for (int tr = 0; tr < T; tr++) {
+			copy_async4(cur_n + tr * 32 + lane, tn_i + (size_t)tr * ncol + cl);
+			copy_async4(cur_m + tr * 32 + lane, mean_i + (size_t)tr * ncol + cl);
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	if ((tid & ~31) < ncol) stage(tid & ~31);
+	for (int col0 = tid & ~31; col0 < ncol; col0 += NT) {
+		const int col = col0 + lane;
+		const bool on = col < ncol;
+		const int cl = on ? col : ncol - 1, c = cl / DP, dp = cl - c * DP;
+		const int st = dp / DPS, dpl = dp - st * DPS, a = s.age[dpl], sc = st * A + c;
+		// (global memory for models whose state does not fit on chip: the loads go out together)
+		int32_t pr[kMaxT];
+#pragma unroll
+		for (int co = 0; co < kMaxT; co++)
+			if (co < C) pr[co] = pc[co * ncol + cl];
+		const float popu_inf = (float)pc[inf_from * ncol + c * DP + dpl];
+#pragma unroll
+		for (int co = 0; co < kMaxT; co++)
+			if (co < C) pv[co * 32] = pr[co];
+		for (int co = kMaxT; co < C; co++) pv[co * 32] = pc[co * ncol + cl];
+		float minf = 0.f;
+		if (popu_inf > 0.f) {
+			const float popu = popu_inf;
+			const float fac = m.M_factor_f[c], dg = m.M_diag_f[c];
+			const float *Ic = Ic_cur + sc * MG, *Im = s.Imap + sc * MG;
+			const float *N = Nm + a * G;
+			float nmi = 0.f;
+#pragma unroll
+			for (int aa = 0; aa < MG; aa++) {
+				if (aa < G) {
+					const float id = Ic[aa] * dg;
+					nmi = fmaf(N[aa], (id + Im[aa]) * d + fac * id * omd, nmi);
+				}
+			}
+			nmi = fmaxf(nmi, 0.f);
+			const float eage = b.nefoi_stage ? s.eage[s.eref[sc] * G + a] : __ldg(tb.efoi_age + (size_t)s.eref[sc] * G + a);
+			minf = dt * popu * s.sus[dp] * (be[sc] * nmi + et[sc] * eage);
+		}
+		const bool fresh = b.simu && b.simu[((size_t)p * m.S + sett) * A + c];   // a SIMU cell
+		int npi = 0, npb = 0, nbi = 0, nbb = 0;              // Poisson / binomial, inversion / rejection
+		asm volatile("cp.async.wait_all;" ::: "memory");     // (each lane reads what it copied itself)
+		for (int tr = 0; tr < T; tr++) {
+			const int id = tr * 32 + lane;
+			float mean;
+			if (tr == itr) mean = minf;
+			else {
+				const float popu = (float)pv[s.from[tr] * 32];
+				mean = popu <= 0.f ? 0.f : dt * popu * s.rate[tr * DP + dp];
+			}
+			if (tb.tm_mult) mean *= __ldg(tb.tm_mult + ((size_t)sett * A + c) * T * DP + tr * DP + dp);
+			const int32_t ni = cur_n[id];
+			const float ri = cur_m[id];
+			if (on) mean_p[(size_t)tr * ncol + cl] = mean;
+			bool pi = false, pb = false, bi = false, bb = false;
+			float v = 0.f;
+			int32_t n = 0;
+			if (mean != mean) atomicCAS(status, 0, BEEP_NAN_RATE);
+			else if (mean > 1.0e9f) atomicCAS(status, 0, BEEP_COUNT_OVERFLOW);
+			else if (mean > 0.f && on) {
+				const bool up = fresh || mean > ri;
+				if (up) {
+					v = fresh ? mean : mean - ri;
+					n = fresh ? 0 : ni;
+					pi = v < 10.f;
+					pb = !pi;
+				} else if (mean == ri) {
+					n = ni;
+				} else if (ni > 0) {
+					v = mean / ri;
+					n = ni;
+					if (!(v > 0.f)) n = 0;
+					else if (v < 1.f) {
+						const float qq = v > 0.5f ? 1.f - v : v;
+						bi = (float)ni * qq < 10.f;
+						bb = !bi;
+					}
+				}
+			}
+			par[id] = v;
+			cnt[id] = n;
+			const unsigned vpi = __ballot_sync(kAll, pi), vpb = __ballot_sync(kAll, pb);
+			const unsigned vbi = __ballot_sync(kAll, bi), vbb = __ballot_sync(kAll, bb);
+			if (pi) lp[npi + __popc(vpi & below)] = (uint8_t)id;
+			if (pb) lp[last - npb - __popc(vpb & below)] = (uint8_t)id;
+			if (bi) lb[nbi + __popc(vbi & below)] = (uint8_t)id;
+			if (bb) lb[last - nbb - __popc(vbb & below)] = (uint8_t)id;
+			npi += __popc(vpi);
+			npb += __popc(vpb);
+			nbi += __popc(vbi);
+			nbb += __popc(vbb);
+		}
+		__syncwarp();
+		if (col0 + NT < ncol) stage(col0 + NT);
+		bool gave_up = false;
+		for (int i = lane; i < npi; i += 32) {
+			const int id = lp[i];
+			cnt[id] += poisson_inversion(par[id], (uint32_t)(col0 + (id & 31)), (uint32_t)(id >> 5), q, s.rcp);
+		}
+		if (npb > 0)
+			ptrs_list(npb, par, (uint32_t)col0, q, s.lnfact, lane, [&](int k) { return (int)lp[last - k]; },
+			          [&](int id, int32_t k) {
+				          cnt[id] = k < 0 ? 0 : cnt[id] + k;
+				          gave_up |= k < 0;
+			          });
+		for (int i = lane; i < nbi + nbb; i += 32) {
+			const int id = i < nbi ? lb[i] : lb[last - (i - nbi)];
+			const int32_t k = binomial_fp32(par[id], cnt[id], q.k0, q.k1, (uint32_t)(col0 + (id & 31)), (uint32_t)(id >> 5),
+			                                q.sett, q.stream, q.lim);
+			cnt[id] = k < 0 ? 0 : k;
+			gave_up |= k < 0;
+		}
+		if (gave_up) atomicCAS(status, 0, BEEP_TIMEOUT);
+		__syncwarp();
+		if (!on) continue;
+		for (int tr = 0; tr < T; tr++) {
+			const int32_t n = cnt[tr * 32 + lane];
+			tn_p[(size_t)tr * ncol + col] = n;
+			const int row = s.trow[tr];
+			if (row >= 0) s.tn[row * ncol + col] = n;
+			pv[s.from[tr] * 32] -= n;
+			pv[s.to[tr] * 32] += n;
+		}
+		float iv = 0.f;
+		for (int co = 0; co < C; co++) {
+			const int32_t v = pv[co * 32];
+			pn[co * ncol + col] = v;
+			const float inf = s.inf[co];
+			if (inf != 0.f) iv = fmaf(inf, (float)v, iv);
+		}
+		if (m.dp_age_unique) Ic_nxt[sc * MG + a] = iv;
+		else atomicAdd(Ic_nxt + sc * MG + a, iv);
+	}
+}
+
 // CTAs resident per SM (MB): one of 640 threads; two to four of 320
 // (kDualThreads) when that many particles' state fits the SM's shared memory
 // -- the register budget per thread shrinks to 96 / 64 / 48 and the warps per
@@ -851,6 +1226,7 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 		s.red = (float *)take(4 * 2 * (size_t)NT);
 		s.mv = NT == kDualThreads ? (float *)take(4 * (size_t)T * NT) : nullptr;
 		s.dn = PD ? (int32_t *)take(4 * (size_t)C * ncol) : nullptr;
+		s.queue = CH && b.ch_queue ? take(chain_queue_bytes(T, C, NT)) : nullptr;
 	}
 	// tensor-core FOI (large models, 640 threads): chunk ring, stacked counts, barriers, tensor memory
 	__shared__ uint64_t tc_bars[2 * tc::kStages + 1];
@@ -962,7 +1338,13 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 
 		// ---- A: per column (c, dp): NMI, means, draws, next population and infectious count
 		const float d = s.dgeo[sb], omd = 1.f - d;
-		for (int col = tid; col < ncol; col += NT) {
+		const bool queued = CH && s.queue && cmode == 1 && !b.simu_all;
+		if constexpr (CH) {
+			if (queued)
+				chain_columns<NT, MG>(m, b, tb, s, p, sett, DrawKey{k0, k1, (uint32_t)sett, stream, lim}, pc, pn, Ic_cur,
+				                      Ic_nxt, be, et, Nm, d, omd, cs_i, cs_p);
+		}
+		for (int col = tid; col < ncol && !queued; col += NT) {
 			const int c = col / DP, dp = col - c * DP;
 			const int st = dp / DPS, dpl = dp - st * DPS, a = s.age[dpl];
 			U4 inv{0, 0, 0, 0};
