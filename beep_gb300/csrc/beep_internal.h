@@ -22,6 +22,7 @@ struct ModelDev {
 	const double *M_diag, *M_factor;
 	const int32_t *csc_ptr, *csc_src;    // [A+1], [nnz]
 	const double *csc_val;               // [nnz]
+	int32_t mix_regular;                 // every csc_val and M_diag is normal, with an exponent within 500
 	const int32_t *pop_init;             // [A][C][DP]
 	// observations
 	const int32_t *obs_model, *obs_kind, *obs_spline, *obs_cell_ptr, *obs_cells, *obs_sett_i, *obs_sett_f;
@@ -110,6 +111,8 @@ struct BatchDev {
 	double *ch_mean;                    // [2][P][S][A][T][DP]
 	double *ch_Imap, *ch_Idiag;         // [2][P][S][NS][A][G]
 	double *Li;                         // [P] mode 2 output
+	const double *lgam;                 // mode 2, plain form: log k! for k < nlgam (launch_lgamma_table)
+	int32_t nlgam;
 	int32_t ch_queue;                   // fast form chains: proposals queue their draws (set by the launchers)
 	float *ch_mean_f;                   // fast form chains: means [2][P][S][T][A*DP] (counts in ch_tn, same layout)
 	// fast form: force of infection on the tensor cores (foi_tc.cuh); its shared
@@ -158,6 +161,8 @@ inline cudaError_t allow_dynamic_smem(K kern, size_t need)
 
 // launchers
 int launch_sim_plain(const ModelDev &m, const BatchDev &b, void *stream);   // sim_plain.cu
+constexpr int kLgammaTable = 4096;               // counts whose log k! a state likelihood looks up
+int launch_lgamma_table(double *t, int n, void *stream);
 int launch_sim_fast(const ModelDev &m, const BatchDev &b, void *stream);    // sim_fast.cu
 size_t fast_smem_bytes(const ModelDev &m, int nslots, bool m_in_smem, int nefoi_stage, bool state_global, int tnrows,
                        bool pop_single, bool tn_smem = false, int nt = 0, int mg = 0,    // mg: age stride (0: G to 4s)

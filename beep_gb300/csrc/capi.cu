@@ -396,6 +396,12 @@ beep_status beep::model_create_internal(const beep_model_desc *d, std::shared_pt
 	md.dp_age = (const int32_t *)(base + o_age); md.M_diag = (const double *)(base + o_diag);
 	md.M_factor = (const double *)(base + o_fac); md.csc_ptr = (const int32_t *)(base + o_cp);
 	md.csc_src = (const int32_t *)(base + o_cs); md.csc_val = (const double *)(base + o_cv);
+	md.mix_regular = 1;
+	auto regular = [](double x) { return std::fabs(x) >= std::ldexp(1.0, -500) && std::fabs(x) <= std::ldexp(1.0, 500); };
+	for (double v : csc_val)
+		if (!regular(v)) md.mix_regular = 0;
+	for (int c = 0; c < A; c++)
+		if (!regular(d->M_diag[c])) md.mix_regular = 0;
 	md.pop_init = (const int32_t *)(base + o_pi);
 	md.obs_model = (const int32_t *)(base + o_om); md.obs_kind = (const int32_t *)(base + o_ok);
 	md.obs_spline = (const int32_t *)(base + o_os); md.obs_cell_ptr = (const int32_t *)(base + o_ocp);

@@ -112,7 +112,7 @@ beep_status prepare_chains(beep_mbp_chains *c, const beep_mbp_request *r, int mo
 	const bool mask = mode == 1 && !simu_all && r->simu;
 	Layout L;
 	const size_t o_cur = L.add((size_t)P), o_simu = L.add(mask ? (size_t)P * m->S * m->A : 0),
-	             o_li = L.add(8 * (size_t)P);
+	             o_li = L.add(8 * (size_t)P), o_lg = L.add(mode == 2 && c->form != BEEP_FORM_FAST ? 8 * (size_t)kLgammaTable : 0);
 	cudaError_t e = c->aux.reserve(L.size);
 	if (e != cudaSuccess) return fail(BEEP_OOM, std::string("chain buffers: ") + cudaGetErrorString(e));
 	char *d = (char *)c->aux.ptr;
@@ -129,6 +129,13 @@ beep_status prepare_chains(beep_mbp_chains *c, const beep_mbp_request *r, int mo
 	bd.ch_tn = c->tn; bd.ch_mean = c->mean; bd.ch_Imap = c->Imap; bd.ch_Idiag = c->Idiag;
 	bd.ch_mean_f = c->mean_f;
 	bd.Li = (double *)(d + o_li);
+	bd.nlgam = 0;
+	if (mode == 2 && c->form != BEEP_FORM_FAST) {
+		bd.lgam = (const double *)(d + o_lg);
+		bd.nlgam = kLgammaTable;
+		const int le = launch_lgamma_table((double *)(d + o_lg), kLgammaTable, m->stream);
+		if (le != 0) return fail(BEEP_DEVICE_ERROR, std::string("log-factorial table: ") + cudaGetErrorString((cudaError_t)le));
+	}
 	st = beep_batch_upload(q);
 	if (st == BEEP_OK) *out = q;
 	return st;

@@ -35,6 +35,7 @@
 //           state (Mbp::parameter_proposal, src/mbp.cc:460-478).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <type_traits>
@@ -159,11 +160,42 @@ __device__ __forceinline__ bool is_nan(double x)
 	return (unsigned long long)(__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ull;
 }
 
+// Integer-valued infectious-count changes (integer infectivities: the counts' sums are integers)
+// are kept as a normalised 32-bit magnitude and {sign, bits}, so that their products with the
+// mixing matrix come from the integer pipe: 20 instructions beside the sum's 64 cycles on the
+// FP64 pipe instead of 64 more on it.  {0, 0} is zero; a magnitude without its top bit marks a
+// value kept as a double.
+__device__ __forceinline__ uint2 encode_int(long long v)
+{
+	const unsigned long long a = (unsigned long long)(v < 0 ? -v : v);
+	if (a == 0) return make_uint2(0u, 0u);
+	if (a >> 32) return make_uint2(1u, 0u);
+	const uint32_t x = (uint32_t)a;
+	const int z = __clz((int)x);
+	return make_uint2(x << z, (v < 0 ? 0x80000000u : 0u) | (uint32_t)(32 - z));
+}
+
+// The IEEE product, rounded to nearest even, of an encoded integer and a normal double of
+// exponent -500 to 500: 53 x 32 bits, the top 53 kept
+__device__ __forceinline__ double mul_int(uint2 d, double v)
+{
+	const uint32_t vh = (uint32_t)__double2hiint(v), vl = (uint32_t)__double2loint(v);
+	const uint64_t lo = (uint64_t)vl * d.x;
+	const uint64_t t = (uint64_t)((vh & 0xfffffu) | 0x100000u) * d.x + (lo >> 32);   // the product / 2^32
+	const uint32_t w = (uint32_t)lo;
+	const bool top = (t >> 52) != 0;
+	uint64_t mant = top ? t : (t << 1) | (w >> 31);
+	const uint32_t rest = top ? w : w << 1;
+	mant += rest > 0x80000000u || (rest == 0x80000000u && (mant & 1u)) ? 1u : 0u;
+	const uint32_t e = ((vh >> 20) & 0x7ffu) + (d.y & 63u) - (top ? 1u : 2u);       // (the mantissa's top bit adds one)
+	return __longlong_as_double((long long)((((uint64_t)e << 52) + mant) | ((uint64_t)((vh ^ d.y) & 0x80000000u) << 32)));
+}
+
 // What the kernel keeps in shared memory: level 2 the particle's arrays and the tables, level 1
 // the tables (a larger model's arrays stay in its global work region), level 0 nothing.
 // The step's tables are double-buffered: a step's are loaded during the previous step's draws.
 struct PlainSmem {
-	size_t pop, tn, imap, idiag, dinf, x, rate, sus, infdif, bea, eta, N, diag, fac, from, to, age, adp, brow, eref, total;
+	size_t pop, tn, imap, idiag, dinf, x, rate, sus, infdif, bea, eta, N, diag, fac, from, to, age, adp, brow, eref, dint, idi, total;
 	__host__ __device__ PlainSmem(const ModelDev &m, int pop_bytes, int level)
 	{
 		size_t off = 0;
@@ -190,19 +222,23 @@ struct PlainSmem {
 		adp = take(4 * (size_t)m.G);
 		brow = take(4 * sa);
 		eref = take(4 * sa);
+		dint = take(8 * ag);
+		idi = take(4 * (size_t)m.T);
 		total = off;
 	}
 };
 
 // One CTA per particle.  Bound: latency of a step's dependent phases for small models; the
 // FP64 pipe (one warp instruction per 16 cycles and SM) for large ones, where the
-// area-mixing sums, two operations per (source, target, age), remain.  Everything else
+// area-mixing sums remain: an addition per (source, target, age), its product formed on the
+// integer pipe where the counts are integers (187 particles of 77x5 over 180 steps: 138 ms with
+// everything on the FP64 pipe, 16.8 ms before the products left it, 12.3 ms now).  The rest
 // was taken off that pipe: the draws are decided in FP32 (rng_filter.cuh), comparisons and
 // zero tests are done on the bits, a target's NMI terms are formed once instead of once
 // per age, unit observation factors sum their integer counts as integers.
 // PopT: int32_t, or double for models with demographic changes.
 template <typename PopT>
-__global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m, const BatchDev b, const int level)
+__global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m, const BatchDev b, const int level, const int sms)
 {
 	constexpr bool kPop64 = sizeof(PopT) == 8;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -210,7 +246,9 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 	const uint32_t lim = b.sampler_limit ? b.sampler_limit : 65536u;   // sampler rejection iterations
 	const int p = blockIdx.x;
 	if (p >= b.P) return;
-	const int tid = threadIdx.x, nth = blockDim.x;
+	// CTAs that share an SM start their threads two schedulers apart: the small models' FP64 work
+	// is one warp's, and two of them on one scheduler took turns on its pipe
+	const int nth = blockDim.x, tid = (threadIdx.x + 64 * ((p / sms) & 1)) & (nth - 1);
 	const int A = m.A, G = m.G, DP = m.DP, NS = m.NS, DPS = m.DPS, C = m.C, T = m.T, ncol = A * DP, GG = G * G;
 	const size_t popsz = (size_t)C * ncol, tnsz = (size_t)T * ncol;
 	const int agsz = NS * A * G, NSA = NS * A;
@@ -265,11 +303,26 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 	const int32_t *from = table(lay.from, m.trans_from, T), *to = table(lay.to, m.trans_to, T);
 	const int32_t *age = table(lay.age, m.dp_age, DPS);
 	const int32_t *brow = table(lay.brow, ip + dir.beta_row_of, NSA), *eref = table(lay.eref, ip + dir.efoi_ref, NSA);
+	uint2 *dint = (uint2 *)(smem_raw + lay.dint);
+	int32_t *idi = (int32_t *)(smem_raw + lay.idi);
+	__shared__ int s_soft;
+	if (tid == 0) {
+		// integer infectivities (and a mixing matrix of ordinary values): dinf as integers
+		bool whole = smem_tabs && m.mix_regular;
+		for (int tr = 0; tr < T && whole; tr++) {
+			const double x = fp[dir.infdif + tr];
+			whole = fabs(x) <= 1024.0 && x == floor(x);
+			idi[tr] = (int32_t)x;
+		}
+		for (int co = 0; co < C && whole; co++) whole = fabs(infectivity[co]) <= 1024.0 && infectivity[co] == floor(infectivity[co]);
+		s_soft = whole;
+	}
 	if (one_dp)
 		for (int dp = tid; dp < DPS; dp += nth) adp[m.dp_age[dp]] = dp;
 	filter_tab_fill(ftab, tid, nth);
 	__syncthreads();
 
+	const bool soft = s_soft != 0;
 	const Div divDP(DP, tnsz + popsz), divG(G, agsz), divA(A, NSA), divDPS(DPS, (size_t)A * DPS);
 	// a step's tables of (strain, area) i: beta * areafactor, external force per capita
 	auto slice = [&](int s, int i, double &be, double &et) {
@@ -291,11 +344,27 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 	auto dinf_of_counts = [&](const int32_t *cnt, const int32_t *base) {
 		for (int idx = tid; idx < agsz; idx += nth) {
 			const int sc = divG.quot(idx), a = idx - sc * G, st = divA.quot(sc), c = sc - st * A;
+			const int dp0 = one_dp ? adp[a] : 0, dp1 = one_dp ? dp0 + 1 : DPS;
+			if (soft) {
+				long long s = 0;
+				for (int tr = 0; tr < T; tr++) {
+					const int di = idi[tr];
+					if (di == 0) continue;
+					for (int dp = dp0; dp < dp1; dp++) {
+						if (age[dp] != a) continue;
+						const int cl = (c * T + tr) * DP + st * DPS + dp;
+						s += (long long)di * (base ? cnt[cl] - base[cl] : cnt[cl]);
+					}
+				}
+				const uint2 q = encode_int(s);
+				dint[idx] = q;
+				if (q.x == 1u) dinf[idx] = (double)s;
+				continue;
+			}
 			double s = 0.0;
 			for (int tr = 0; tr < T; tr++) {
 				const double di = infdif[tr];
 				if (is_zero(di)) continue;
-				const int dp0 = one_dp ? adp[a] : 0, dp1 = one_dp ? dp0 + 1 : DPS;
 				for (int dp = dp0; dp < dp1; dp++) {
 					if (age[dp] != a) continue;
 					const int cl = (c * T + tr) * DP + st * DPS + dp;
@@ -343,6 +412,7 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 					}
 				}
 				dinf[idx] = s;
+				if (soft) dint[idx] = is_zero(s) ? make_uint2(0u, 0u) : make_uint2(1u, 0u);
 			}
 			__syncthreads();
 		}
@@ -361,10 +431,22 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 				const double *dst = dinf + (size_t)st * A * G + a;
 				double im = sett == b.ti ? 0.0 : Imap[idx];
 				double id = sett == b.ti ? 0.0 : Idiag[idx];
-				if (!(dif && sett == b.ti)) {
+				const int j1 = m.csc_ptr[t + 1];
+				if (dif && sett == b.ti) {
+				} else if (soft) {
+					const uint2 *dq = dint + (size_t)st * A * G + a;
+					const uint2 q = dq[t * G];
+					if (q.x != 0u) id += q.x == 1u ? dst[t * G] * diag[t] : mul_int(q, diag[t]);
+#pragma unroll 4
+					for (int j = m.csc_ptr[t]; j < j1; j++) {
+						const int src = m.csc_src[j] * G;
+						const double v = m.csc_val[j];
+						const uint2 qs = dq[src];
+						if (qs.x != 0u) im += qs.x == 1u ? dst[src] * v : mul_int(qs, v);
+					}
+				} else {
 					const double dself = dst[t * G];
 					if (!is_zero(dself)) id += dself * diag[t];
-					const int j1 = m.csc_ptr[t + 1];
 #pragma unroll 4
 					for (int j = m.csc_ptr[t]; j < j1; j++) {
 						const double ds = dst[m.csc_src[j] * G], v = m.csc_val[j];
@@ -455,9 +537,14 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 			if (mode >= 2) {                    // the given counts stay
 				n = ext[cell];
 				if (mode == 2) {                  // State::likelihood term of the fixed count
-					const double lp = poisson_lp(n, mean);
+					double lp;
+					// (no logarithm for a zero count, log n! from the table: the same values)
+					if (n == 0 && (unsigned long long)__double_as_longlong(mean) < 0x7ff0000000000000ull) lp = -mean;
+					else if (n <= 0 || n >= b.nlgam || is_zero(mean)) lp = poisson_lp(n, mean);
+					else lp = n * log(mean) - mean - b.lgam[n];
 					const double t = Lsum + lp;
-					Lcmp += fabs(Lsum) >= fabs(lp) ? (Lsum - t) + lp : (lp - t) + Lsum;
+					const bool big = (__double_as_longlong(Lsum) & 0x7fffffffffffffffll) >= (__double_as_longlong(lp) & 0x7fffffffffffffffll);
+					Lcmp += ((big ? Lsum : lp) - t) + (big ? lp : Lsum);
 					Lsum = t;
 				} else {
 					b.ch_mean[chs(cs_p, sett) * tnsz + cell] = mean;
@@ -631,6 +718,12 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 
 namespace {
 
+__global__ void __launch_bounds__(256) lgamma_table(double *t, int n)
+{
+	const int k = blockIdx.x * 256 + threadIdx.x;
+	if (k < n) t[k] = lgamma((double)(k + 1));
+}
+
 template <typename PopT>
 int launch_pop(const ModelDev &m, const BatchDev &b, cudaStream_t st)
 {
@@ -647,11 +740,17 @@ int launch_pop(const ModelDev &m, const BatchDev &b, cudaStream_t st)
 	if (e == cudaSuccess) e = allow_dynamic_smem(sim_plain_kernel<PopT>, smem);
 	if (e != cudaSuccess) return (int)e;
 	const int nth = b.P <= sms && m.T * m.A * m.DP > 256 ? 512 : 256;
-	sim_plain_kernel<PopT><<<b.P, nth, smem, st>>>(m, b, level);
+	sim_plain_kernel<PopT><<<b.P, nth, smem, st>>>(m, b, level, std::max(1, sms));
 	return (int)cudaGetLastError();
 }
 
 }  // namespace
+
+int launch_lgamma_table(double *t, int n, void *stream)
+{
+	lgamma_table<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(t, n);
+	return (int)cudaGetLastError();
+}
 
 int launch_sim_plain(const ModelDev &m, const BatchDev &b, void *stream)
 {
