@@ -324,13 +324,25 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 
 	const bool soft = s_soft != 0;
 	const Div divDP(DP, tnsz + popsz), divG(G, agsz), divA(A, NSA), divDPS(DPS, (size_t)A * DPS);
-	// a step's tables of (strain, area) i: beta * areafactor, external force per capita
-	auto slice = [&](int s, int i, double &be, double &et) {
+	// a step's tables of (strain, area) i: beta * areafactor, external force per capita (loaded, and
+	// combined once the loads have landed)
+	auto slice_load = [&](int s, int i, double &be, double &af, double &et, double &em) {
 		const int st = divA.quot(i), c = i - st * A;
-		be = beta_rows[(size_t)brow[i] * m.S + s] * areafactor[(size_t)(s / m.div_per_time) * A + c];
+		be = beta_rows[(size_t)brow[i] * m.S + s];
+		af = areafactor[(size_t)(s / m.div_per_time) * A + c];
 		et = efoi_spline[(size_t)eref[i] * m.S + s];
+		if (efoi_mult) em = efoi_mult[((size_t)s * A + c) * NS + st];
+	};
+	auto slice_value = [&](double be, double af, double et, double em, double &b_out, double &e_out) {
+		b_out = be * af;
 		if (!is_zero(et)) et = et / m.popsize;
-		if (efoi_mult) et *= efoi_mult[((size_t)s * A + c) * NS + st];
+		if (efoi_mult) et *= em;
+		e_out = et;
+	};
+	auto slice = [&](int s, int i, double &be, double &et) {
+		double q0, q1, q2, q3 = 1.0;
+		slice_load(s, i, q0, q1, q2, q3);
+		slice_value(q0, q1, q2, q3, be, et);
 	};
 	for (int i = tid; smem_tabs && i < NSA; i += nth) slice(b.ti, i, bea[i], eta[i]);
 	for (int i = tid; smem_tabs && i < GG; i += nth) Nm[i] = Ntime[(size_t)b.ti * GG + i];
@@ -341,8 +353,9 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 	const int cols = (T * pad + nth - 1) / nth <= ((int)tnsz + nth - 1) / nth ? pad : ncol;
 	const Div divCol(cols, (size_t)T * cols);
 	// dinf per (strain, source area, age) of the next step's maps, from the step's counts
+	const int tinf = (tid + 32) & (nth - 1);             // (the last warp first: see below)
 	auto dinf_of_counts = [&](const int32_t *cnt, const int32_t *base) {
-		for (int idx = tid; idx < agsz; idx += nth) {
+		for (int idx = tinf; idx < agsz; idx += nth) {
 			const int sc = divG.quot(idx), a = idx - sc * G, st = divA.quot(sc), c = sc - st * A;
 			const int dp0 = one_dp ? adp[a] : 0, dp1 = one_dp ? dp0 + 1 : DPS;
 			if (soft) {
@@ -378,8 +391,16 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 
 	const int itr = m.infection_trans;
 	const int inf_from = m.trans_from[itr];
+	// Loads whose latency a small model's step would wait for are issued a phase or a step ahead,
+	// by the threads that draw last: the tables of the next step by the last warps (tslice), the
+	// observations from three quarters of the CTA on (tobs), the next infectious changes by the
+	// last warp first (tinf).
+	const int tslice = nth - 1 - tid, tobs = (tid + nth / 4) & (nth - 1);
+	const bool few = agsz <= nth / 4;
 	int buf = 0;
-	int opos = b.step_ptr[0] + tid < b.step_ptr[1] ? b.step_obs[b.step_ptr[0] + tid] : 0;   // this thread's first observation
+	int s0 = b.step_ptr[0], s1 = b.step_ptr[1], s2 = b.step_ptr[min(2, nsteps)];   // this step's observations and the next's
+	int opos = s0 + tobs < s1 ? b.step_obs[s0 + tobs] : 0;   // this thread's first observation
+	double d_next = geo[b.ti];
 	for (int sett = b.ti; sett < b.tf; sett++) {
 		// the step's counts: in shared memory, or the output or chain array itself (ext)
 		int32_t *ext = mode ? b.ch_tn + chs(writes ? cs_p : cs_i, sett) * tnsz
@@ -389,9 +410,23 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 		const double *be = bea + buf * NSA, *et = eta + buf * NSA;
 		const double *N = smem_tabs ? Nm + buf * GG : Ntime + (size_t)sett * GG;
 		const int sn = sett + 1 < b.tf ? sett + 1 : sett;
-		const double d = geo[sett], omd = 1 - d;
-		const int s0 = b.step_ptr[sett - b.ti], s1 = mode == 2 ? s0 : b.step_ptr[sett - b.ti + 1];
-		const int oidx = s0 + tid < s1 ? b.scored[opos] : -1;
+		const double d = d_next, omd = 1 - d;
+		d_next = geo[sn];
+		const bool scoring = mode != 2;
+		const int s3 = b.step_ptr[min(sett + 3 - b.ti, nsteps)];
+		const int oidx = scoring && s0 + tobs < s1 ? b.scored[opos] : -1;
+		// the current state's cell of this thread's first draw (MBP chains)
+		int32_t first_n = 0;
+		double first_r = 0.0;
+		if (mode == 1 && !b.simu_all && tid < T * cols) {
+			const int tr = divCol.quot(tid), col = tid - tr * cols;
+			if (col < ncol) {
+				const int c = divDP.quot(col);
+				const size_t ci = chs(cs_i, sett) * tnsz + ((size_t)c * T + tr) * DP + (col - c * DP);
+				first_n = b.ch_tn[ci];
+				first_r = b.ch_mean[ci];
+			}
+		}
 
 		if constexpr (kPop64) {
 			if (m.ndcc > 0) democat_adjust(m, pop_cur, sett, tid, nth);   // pop[sett] before its step
@@ -424,9 +459,10 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 			const int sc = divG.quot(idx), a = idx - sc * G, st = divA.quot(sc), t = sc - st * A;
 			double imv, idv;                               // the state's maps
 			const size_t io = mode ? chs(cs_i, sett) * agsz + idx : 0;
+			const double im_i = dif || mode == 2 ? b.ch_Imap[io] : 0.0, id_i = dif || mode == 2 ? b.ch_Idiag[io] : 0.0;
 			if (mode == 2) {
-				imv = b.ch_Imap[io];
-				idv = b.ch_Idiag[io];
+				imv = im_i;
+				idv = id_i;
 			} else {
 				const double *dst = dinf + (size_t)st * A * G + a;
 				double im = sett == b.ti ? 0.0 : Imap[idx];
@@ -437,8 +473,41 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 					const uint2 *dq = dint + (size_t)st * A * G + a;
 					const uint2 q = dq[t * G];
 					if (q.x != 0u) id += q.x == 1u ? dst[t * G] * diag[t] : mul_int(q, diag[t]);
+					// few elements: four products at once (independent), then their additions in order;
+					// many: the warps hide each other, and zero counts are passed by (77 areas x 5 ages:
+					// 13.8 ms with four at once against 12.3 ms; 10 x 3: 4.6 against 4.9 ms)
+					int j = m.csc_ptr[t];
+					for (; few && j + 4 <= j1; j += 4) {
+						uint2 qs[4];
+						double v[4];
+						bool wide = false;
+#pragma unroll
+						for (int u = 0; u < 4; u++) {
+							qs[u] = dq[m.csc_src[j + u] * G];
+							v[u] = m.csc_val[j + u];
+							wide |= qs[u].x == 1u;
+						}
+						if (!wide) {
+#pragma unroll
+							for (int u = 0; u < 4; u++) v[u] = mul_int(qs[u], v[u]);
+						} else {
+#pragma unroll 1
+							for (int u = 0; u < 4; u++) {
+								const uint2 q1 = u == 0 ? qs[0] : u == 1 ? qs[1] : u == 2 ? qs[2] : qs[3];
+								const double v1 = u == 0 ? v[0] : u == 1 ? v[1] : u == 2 ? v[2] : v[3];
+								const double pr = q1.x == 1u ? dst[m.csc_src[j + u] * G] * v1 : mul_int(q1, v1);
+								if (u == 0) v[0] = pr;
+								else if (u == 1) v[1] = pr;
+								else if (u == 2) v[2] = pr;
+								else v[3] = pr;
+							}
+						}
+#pragma unroll
+						for (int u = 0; u < 4; u++)
+							if (qs[u].x != 0u) im += v[u];
+					}
 #pragma unroll 4
-					for (int j = m.csc_ptr[t]; j < j1; j++) {
+					for (; j < j1; j++) {
 						const int src = m.csc_src[j] * G;
 						const double v = m.csc_val[j];
 						const uint2 qs = dq[src];
@@ -455,8 +524,8 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 				}
 				Imap[idx] = im;
 				Idiag[idx] = id;
-				imv = dif ? b.ch_Imap[io] + im : im;
-				idv = dif ? b.ch_Idiag[io] + id : id;
+				imv = dif ? im_i + im : im;
+				idv = dif ? id_i + id : id;
 				if (writes) {
 					const size_t ow = chs(cs_p, sett) * agsz + idx;
 					b.ch_Imap[ow] = imv;
@@ -488,9 +557,9 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 
 		// ---- D: transition means and counts per (transition, column); the next step's tables
 		// and this thread's next observation are loaded on the way
-		double nbe = 0.0, net = 0.0, nN = 0.0;
-		if (smem_tabs && tid < NSA) slice(sn, tid, nbe, net);
-		if (smem_tabs && tid < GG) nN = Ntime[(size_t)sn * GG + tid];
+		double nb = 0.0, na = 0.0, ne = 0.0, nm = 1.0, nN = 0.0;
+		if (smem_tabs && tslice < NSA) slice_load(sn, tslice, nb, na, ne, nm);
+		if (smem_tabs && tslice < GG) nN = Ntime[(size_t)sn * GG + tslice];
 		int oq0 = 0, oq1 = 0, ospl = -1;
 		double ofac = 0.0, oacc = 0.0;
 		if (oidx >= 0) {
@@ -500,8 +569,7 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 			ofac = m.obs_factor[oidx];
 			oacc = acc[opos];
 		}
-		const int s2 = sett + 1 < b.tf && mode != 2 ? b.step_ptr[sett + 2 - b.ti] : s1;
-		const int npos = s1 + tid < s2 ? b.step_obs[s1 + tid] : 0;
+		const int npos = scoring && s1 + tobs < s2 ? b.step_obs[s1 + tobs] : 0;
 		for (int item = tid; item < T * cols; item += nth) {
 			const int tr = divCol.quot(item), col = item - tr * cols;
 			if (col >= ncol) continue;
@@ -563,8 +631,8 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 					if (mode != 0 && !b.simu_all && !(b.simu && b.simu[((size_t)p * m.S + sett) * A + c])) {
 						// coupled to the current state (src/mbp.cc:293-305)
 						const size_t ci = chs(cs_i, sett) * tnsz + cell;
-						n0 = b.ch_tn[ci];
-						ri = b.ch_mean[ci];
+						n0 = item == tid ? first_n : b.ch_tn[ci];
+						ri = item == tid ? first_r : b.ch_mean[ci];
 						draw = mean - ri;
 						thin = mean < ri;
 					}
@@ -581,19 +649,23 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 			if (copy) ext[cell] = n;
 		}
 		if (smem_tabs) {
-			double *nb = bea + (buf ^ 1) * NSA, *ne = eta + (buf ^ 1) * NSA, *nn = Nm + (buf ^ 1) * GG;
-			if (tid < NSA) { nb[tid] = nbe; ne[tid] = net; }
-			if (tid < GG) nn[tid] = nN;
-			for (int i = tid + nth; i < NSA; i += nth) slice(sn, i, nb[i], ne[i]);
-			for (int i = tid + nth; i < GG; i += nth) nn[i] = Ntime[(size_t)sn * GG + i];
+			double *tb = bea + (buf ^ 1) * NSA, *te = eta + (buf ^ 1) * NSA, *tN = Nm + (buf ^ 1) * GG;
+			if (tslice < NSA) slice_value(nb, na, ne, nm, tb[tslice], te[tslice]);
+			if (tslice < GG) tN[tslice] = nN;
+			for (int i = tslice + nth; i < NSA; i += nth) slice(sn, i, tb[i], te[i]);
+			for (int i = tslice + nth; i < GG; i += nth) tN[i] = Ntime[(size_t)sn * GG + i];
 		}
+		int oc[4];                                           // its first cells
+#pragma unroll
+		for (int i = 0; i < 4; i++) oc[i] = oq0 + i < oq1 ? m.obs_cells[oq0 + i] : 0;
 		__syncthreads();
 
 		// ---- E: observation sums (one thread per active observation, cells in reference order)
-		for (int k = s0 + tid; k < s1; k += nth) {
+		for (int k = scoring ? s0 + tobs : s1; k < s1; k += nth) {
+			const bool head = k == s0 + tobs;
 			int q0 = oq0, q1 = oq1, spl = ospl, pos = opos;
 			double fac = ofac, v = oacc;
-			if (k != s0 + tid) {
+			if (!head) {
 				pos = b.step_obs[k];
 				const int o = b.scored[pos];
 				q0 = m.obs_cell_ptr[o];
@@ -605,7 +677,14 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 			if (!kPop64 && spl < 0 && __double_as_longlong(fac) == __double_as_longlong(1.0)) {
 				// a unit factor: the counts' sum is an integer, exact in either arithmetic
 				long long sum = 0;
-				for (int q = q0; q < q1; q++) {
+				int q = q0;
+				if (head) {
+#pragma unroll
+					for (int i = 0; i < 4; i++)
+						if (q0 + i < q1) sum += oc[i] >= 0 ? (long long)tn[oc[i]] : (long long)pop_cur[-1 - oc[i]];
+					q = q0 + 4;
+				}
+				for (; q < q1; q++) {
 					const int cell = m.obs_cells[q];
 					sum += cell >= 0 ? (long long)tn[cell] : (long long)pop_cur[-1 - cell];
 				}
@@ -627,6 +706,9 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 			acc[pos] = v;
 		}
 		opos = npos;
+		s0 = s1;
+		s1 = s2;
+		s2 = s3;
 		// update_pop into the other buffer, a column per thread and compartment
 		for (int k = tid; k < (int)popsz; k += nth) {
 			const int cc = divDP.quot(k), dp = k - cc * DP, c = cc / C, co = cc - c * C;
