@@ -481,84 +481,122 @@ __global__ void __launch_bounds__(kBxStepThreads, MB) bx_step(const ModelDev m, 
 	}
 }
 
-// The step's observation terms of particle p (completed observations -> log-density,
-// compensated per thread), then the next step's strain shift; with several dp per age
+// The step's observation terms of KP particles (completed observations -> log-density,
+// compensated per thread), then their next step's strain shift; with several dp per age
 // the next infectious counts are accumulated by atomics, so the buffer the step after
 // next accumulates into is cleared here.
+// Bound: latency and the L2 reads of the task records, 32 bytes per particle, task and step
+// where each particle reads them itself, as many as the counts they select.  A CTA of four
+// particles reads a task and its observation's constants once and has four particles' slots
+// and counts in flight (16384 x 150x4: 58 ms of a generation with a CTA per particle, 43 ms now); each
+// particle's terms keep their threads and order.
+template <int KP>
 __global__ void __launch_bounds__(kBxObsThreads) bx_obs(const ModelDev m, const BatchDev b, int sett)
 {
-	const int p = blockIdx.x, tid = threadIdx.x;
+	const int p0 = blockIdx.x * KP, np_ = min(KP, b.P - p0), tid = threadIdx.x;
 	const int A = m.A, G = m.G, NS = m.NS, ncol = A * m.DP;
 	const int tnrows = b.tn_full ? m.T : m.tn_rows;
 	const int s_rel = sett - b.ti, cur = s_rel & 1;
-	const Tabs tb = bx_tabs(b, p);
-	const int32_t *pc = bx_pop(m, b, p, cur);
-	const int32_t *tn = b.bx_tn + (size_t)p * tnrows * ncol;
-	float *slot = b.bx_slot + (size_t)p * b.nslots;
-	float2 kah = b.bx_kahan[(size_t)p * kBxObsThreads + tid];
-	float Lsum = kah.x, Lcmp = kah.y;
+	const int32_t *pc[KP], *tn[KP];
+	float *slot[KP];
+	float2 kah[KP];
+	float Lsum[KP], Lcmp[KP];
+#pragma unroll
+	for (int i = 0; i < KP; i++) {
+		const int p = p0 + min(i, np_ - 1);              // (a missing particle reads the last one's)
+		pc[i] = bx_pop(m, b, p, cur);
+		tn[i] = b.bx_tn + (size_t)p * tnrows * ncol;
+		slot[i] = b.bx_slot + (size_t)p * b.nslots;
+		kah[i] = b.bx_kahan[(size_t)p * kBxObsThreads + tid];
+		Lsum[i] = kah[i].x;
+		Lcmp[i] = kah[i].y;
+	}
 	const int a0 = b.step_ptr[s_rel], a1 = b.step_ptr[s_rel + 1];
-	// one task ahead: the next task's record, slot and first cell are loaded before the
+	// one task ahead: the next task's record, slots and first cells are loaded before the
 	// current one is summed (the observations active at a step have distinct slots); each
-	// task's sum and the thread's log-density sum keep their order
-	auto first_of = [&](const int4 &q0) {
+	// task's sum and the thread's log-density sums keep their order
+	auto first_of = [&](const int4 &q0, int i) {
 		const int cell = q0.z;
-		return (q0.w & 0x7fffffff) > 0 ? (cell >= 0 ? (float)tn[cell] : (float)pc[-1 - cell]) : 0.f;
+		return (q0.w & 0x7fffffff) > 0 ? (cell >= 0 ? (float)tn[i][cell] : (float)pc[i][-1 - cell]) : 0.f;
 	};
 	int k = a0 + tid;
 	int4 n0 = make_int4(0, 0, 0, 0), n1 = make_int4(0, 0, 0, 0);
-	float nv = 0.f, nf = 0.f;
-	if (k < a1) {
-		n0 = __ldg(b.tasks + 2 * k);
-		n1 = __ldg(b.tasks + 2 * k + 1);
-		nv = slot[n0.x];
-		nf = first_of(n0);
-	}
+	float nv[KP], nf[KP];
+	auto fetch = [&](int at) {
+		n0 = __ldg(b.tasks + 2 * at);
+		n1 = __ldg(b.tasks + 2 * at + 1);
+#pragma unroll
+		for (int i = 0; i < KP; i++) {
+			nv[i] = slot[i][n0.x];
+			nf[i] = first_of(n0, i);
+		}
+	};
+	if (k < a1) fetch(k);
 	for (; k < a1; k += kBxObsThreads) {
 		const int4 q0 = n0, q1 = n1;
-		float x = nv;
-		const float f = nf;
-		const int kn = k + kBxObsThreads;
-		if (kn < a1) {
-			n0 = __ldg(b.tasks + 2 * kn);
-			n1 = __ldg(b.tasks + 2 * kn + 1);
-			nv = slot[n0.x];
-			nf = first_of(n0);
+		float x[KP], f[KP];
+#pragma unroll
+		for (int i = 0; i < KP; i++) {
+			x[i] = nv[i];
+			f[i] = nf[i];
 		}
+		if (k + kBxObsThreads < a1) fetch(k + kBxObsThreads);
 		const float fac = __int_as_float(q1.x);
-		const int spl = q1.y;
-		const float w = spl < 0 ? fac : fac * tb.obs_spline[(size_t)spl * m.S + sett];
-		const int nc = q0.w & 0x7fffffff;
-		if (nc > 0) x = fmaf(w, f, x);
-		if (q1.w != 0) {                  // consecutive counts or populations: no cell list
-			const int32_t *src = q1.w == 1 ? tn + q0.z : pc + (-1 - q0.z);
+		const int spl = q1.y, nc = q0.w & 0x7fffffff;
+		int kind = BEEP_OBSVAL_UNKNOWN, model = 0;
+		float2 np = make_float2(0.f, 0.f);
+		float value = 0.f;
+		if (q0.w < 0) {                  // the observation's last step: its constants, once for the particles
+			kind = m.obs_kind[q0.y];
+			model = m.obs_model[q0.y];
+			np = m.obs_np[q0.y];
+			value = m.obs_value_f[q0.y];
+		}
+#pragma unroll
+		for (int i = 0; i < KP; i++) {
+			const float w = spl < 0 ? fac : fac * bx_tabs(b, p0 + min(i, np_ - 1)).obs_spline[(size_t)spl * m.S + sett];
+			if (nc > 0) x[i] = fmaf(w, f[i], x[i]);
+			if (q1.w != 0) {                  // consecutive counts or populations: no cell list
+				const int32_t *src = q1.w == 1 ? tn[i] + q0.z : pc[i] + (-1 - q0.z);
 #pragma unroll 4
-			for (int i = 1; i < nc; i++) x = fmaf(w, (float)src[i], x);
-		} else {
-			for (int i = 1; i < nc; i++) {
-				const int cell = __ldg((b.tn_full ? m.obs_cells_full : m.obs_cells_f) + q1.z + i);
-				x = fmaf(w, cell >= 0 ? (float)tn[cell] : (float)pc[-1 - cell], x);
+				for (int j = 1; j < nc; j++) x[i] = fmaf(w, (float)src[j], x[i]);
+			} else {
+				for (int j = 1; j < nc; j++) {
+					const int cell = __ldg((b.tn_full ? m.obs_cells_full : m.obs_cells_f) + q1.z + j);
+					x[i] = fmaf(w, cell >= 0 ? (float)tn[i][cell] : (float)pc[i][-1 - cell], x[i]);
+				}
 			}
+			if (q0.w < 0) {
+				float lp;
+				if (kind == BEEP_OBSVAL_VALUE && (model == BEEP_OBS_NORMAL || model == BEEP_OBS_NORMAL_PERCENT)) {
+					const float d = value - (x[i] < 0.f ? 0.f : x[i]);
+					lp = np.x - d * d * np.y;
+				} else {
+					lp = obs_lp_fast(x[i], q0.y, m);
+				}
+				x[i] = 0.f;
+				const float y = lp - Lcmp[i];      // Kahan
+				const float tt = Lsum[i] + y;
+				Lcmp[i] = (tt - Lsum[i]) - y;
+				Lsum[i] = tt;
+			}
+			if (i < np_) slot[i][q0.x] = x[i];
 		}
-		if (q0.w < 0) {                  // the observation's last step: log-density
-			const float lp = obs_lp_fast(x, q0.y, m);
-			x = 0.f;
-			const float y = lp - Lcmp;      // Kahan
-			const float tt = Lsum + y;
-			Lcmp = (tt - Lsum) - y;
-			Lsum = tt;
-		}
-		slot[q0.x] = x;
 	}
-	if (Lsum != kah.x || Lcmp != kah.y) b.bx_kahan[(size_t)p * kBxObsThreads + tid] = make_float2(Lsum, Lcmp);
+#pragma unroll
+	for (int i = 0; i < KP; i++)
+		if (i < np_ && (Lsum[i] != kah[i].x || Lcmp[i] != kah[i].y))
+			b.bx_kahan[(size_t)(p0 + i) * kBxObsThreads + tid] = make_float2(Lsum[i], Lcmp[i]);
 	if (sett + 1 < b.tf) {
-		// the next product's operand from the counts the step kernel left for the next step
-		bx_pack_a(m, b, p, b.bx_ic + (size_t)(cur ^ 1) * b.P * NS * A * G + (size_t)p * NS * A * G, tid,
-		          kBxObsThreads);
-		if (NS > 1) strain_shift(m, bx_pop(m, b, p, cur ^ 1), tid, kBxObsThreads);
-		if (!m.dp_age_unique) {
-			float *Ic = b.bx_ic + (size_t)cur * b.P * NS * A * G + (size_t)p * NS * A * G;
-			for (int k = tid; k < NS * A * G; k += kBxObsThreads) Ic[k] = 0.f;
+		for (int p = p0; p < p0 + np_; p++) {
+			// the next product's operand from the counts the step kernel left for the next step
+			bx_pack_a(m, b, p, b.bx_ic + (size_t)(cur ^ 1) * b.P * NS * A * G + (size_t)p * NS * A * G, tid,
+			          kBxObsThreads);
+			if (NS > 1) strain_shift(m, bx_pop(m, b, p, cur ^ 1), tid, kBxObsThreads);
+			if (!m.dp_age_unique) {
+				float *Ic = b.bx_ic + (size_t)cur * b.P * NS * A * G + (size_t)p * NS * A * G;
+				for (int j = tid; j < NS * A * G; j += kBxObsThreads) Ic[j] = 0.f;
+			}
 		}
 	}
 }
@@ -620,6 +658,8 @@ int launch_steps(const ModelDev &m, const BatchDev &b, size_t smem_step, int sms
 	const int grid = std::min(nitem, grid0);
 	e = cudaMemsetAsync(b.bx_a, 0, batched_a_bytes(m, b.P), st);   // padding rows and sources stay zero
 	if (e != cudaSuccess) return (int)e;
+	// four particles per observation CTA where that still leaves four CTAs per SM
+	const bool four = b.P >= 16 * sms;
 	bx_init<<<b.P, 256, 0, st>>>(m, b);
 	for (int s = b.ti; s < b.tf; s++) {
 		cudaEvent_t *e4 = ev ? ev + 4 * (s - b.ti) : nullptr;   // before and after each of the step's kernels
@@ -628,7 +668,8 @@ int launch_steps(const ModelDev &m, const BatchDev &b, size_t smem_step, int sms
 		if (e4) cudaEventRecord(e4[1], st);
 		kstep<<<grid, kBxStepThreads, smem_step, st>>>(m, b, s, chunk);
 		if (e4) cudaEventRecord(e4[2], st);
-		bx_obs<<<b.P, kBxObsThreads, 0, st>>>(m, b, s);
+		if (four) bx_obs<4><<<(b.P + 3) / 4, kBxObsThreads, 0, st>>>(m, b, s);
+		else bx_obs<1><<<b.P, kBxObsThreads, 0, st>>>(m, b, s);
 		if (e4) cudaEventRecord(e4[3], st);
 	}
 	bx_final<<<b.P, 256, 0, st>>>(m, b);
