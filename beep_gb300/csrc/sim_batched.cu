@@ -311,8 +311,10 @@ __global__ void __launch_bounds__(256) bx_init(const ModelDev m, const BatchDev 
 // the step's counter.  Per column (c, dp): NMI, the transition means, the keyed draws
 // and the population update, then the column's infectious count for the next step;
 // the counts of observed transitions go to the step's count buffer.
-template <int MG, int MB>
-__global__ void __launch_bounds__(kBxStepThreads, MB) bx_step(const ModelDev m, const BatchDev b, int sett, int chunk)
+// KEYED: each particle has its own Philox key (packed requests); otherwise the batch's is ks.
+template <int MG, int MB, bool KEYED>
+__global__ void __launch_bounds__(kBxStepThreads, MB) bx_step(const ModelDev m, const BatchDev b,
+                                                             const __grid_constant__ KeySched ks, int sett, int chunk)
 {
 	constexpr int NT = kBxStepThreads;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -397,7 +399,7 @@ __global__ void __launch_bounds__(kBxStepThreads, MB) bx_step(const ModelDev m, 
 			__syncthreads();
 		}
 		const uint32_t stream = b.stream_of ? b.stream_of[p] : (uint32_t)p;
-		const uint32_t k0 = b.key_of ? b.key_of[p].x : b.k0, k1 = b.key_of ? b.key_of[p].y : b.k1;
+		const uint2 own = KEYED ? b.key_of[p] : make_uint2(0u, 0u);
 		int32_t *status = b.status + p;
 		const int32_t *pc = bx_pop(m, b, p, cur);
 		int32_t *pn = bx_pop(m, b, p, cur ^ 1);
@@ -456,8 +458,12 @@ __global__ void __launch_bounds__(kBxStepThreads, MB) bx_step(const ModelDev m, 
 				if (mean > 0.f) {
 					if (mean > 1.0e9f) atomicCAS(status, 0, BEEP_COUNT_OVERFLOW);
 					else {
-						n = poisson_fp32(mean, k0, k1, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, inv, inv_call,
-						                 rcp, lnfact, lim);
+						if constexpr (KEYED)
+							n = poisson_fp32(mean, KeyRegs{own.x, own.y}, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, inv,
+							                 inv_call, rcp, lnfact, lim);
+						else
+							n = poisson_fp32(mean, ks, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, inv, inv_call, rcp,
+							                 lnfact, lim);
 						if (n < 0) { atomicCAS(status, 0, BEEP_TIMEOUT); n = 0; }
 					}
 				} else if (mean != mean) atomicCAS(status, 0, BEEP_NAN_RATE);
@@ -635,7 +641,12 @@ __global__ void __launch_bounds__(256) bx_final(const ModelDev m, const BatchDev
 template <int MG, int MB>
 int launch_steps(const ModelDev &m, const BatchDev &b, size_t smem_step, int sms, cudaStream_t st, cudaEvent_t *ev)
 {
-	auto kstep = bx_step<MG, MB>;
+	auto kstep = b.key_of ? bx_step<MG, MB, true> : bx_step<MG, MB, false>;
+	KeySched ks;
+	for (uint32_t r = 0; r < 10; r++) {
+		ks.k0[r] = b.k0 + r * 0x9E3779B9u;
+		ks.k1[r] = b.k1 + r * 0xBB67AE85u;
+	}
 	cudaError_t e = allow_dynamic_smem(kstep, smem_step);
 	if (e != cudaSuccess) return (int)e;
 	const BxGeom x = bx_geometry(m.A, m.NS);
@@ -666,7 +677,7 @@ int launch_steps(const ModelDev &m, const BatchDev &b, size_t smem_step, int sms
 		if (e4) cudaEventRecord(e4[0], st);
 		bx_foi<<<ntile, kBxThreads, smem_foi, st>>>(m, b);
 		if (e4) cudaEventRecord(e4[1], st);
-		kstep<<<grid, kBxStepThreads, smem_step, st>>>(m, b, s, chunk);
+		kstep<<<grid, kBxStepThreads, smem_step, st>>>(m, b, ks, s, chunk);
 		if (e4) cudaEventRecord(e4[2], st);
 		if (four) bx_obs<4><<<(b.P + 3) / 4, kBxObsThreads, 0, st>>>(m, b, s);
 		else bx_obs<1><<<b.P, kBxObsThreads, 0, st>>>(m, b, s);

@@ -102,25 +102,48 @@ __device__ __forceinline__ float ptrs_rhs(float k, float mean, float loglam, con
 	return k * (log1pf(x) - x) - x - 0.5f * __logf(n) - 0.91893853f - corr;
 }
 
+// The Philox blocks of a particle's key, kept in two registers, or of a batch's one key, whose
+// ten round keys a kernel reads from its parameters as operands (20 additions per block less:
+// step kernel of 16384 x 150x4 301 -> 295 ms, of 1024 x 350x10 371 -> 364 ms)
+struct KeyRegs {
+	uint32_t k0, k1;
+	__device__ __forceinline__ U4 operator()(const U4 &c) const { return philox10(c, k0, k1); }
+};
+
+struct KeySched {
+	uint32_t k0[10], k1[10];
+	__device__ __forceinline__ U4 operator()(U4 c) const
+	{
+#pragma unroll
+		for (int r = 0; r < 10; r++) {
+			const uint32_t lo0 = 0xD2511F53u * c.x, hi0 = __umulhi(0xD2511F53u, c.x);
+			const uint32_t lo1 = 0xCD9E8D57u * c.z, hi1 = __umulhi(0xCD9E8D57u, c.z);
+			c = U4{hi1 ^ c.y ^ k0[r], lo1, hi0 ^ c.w ^ k1[r], lo0};
+		}
+		return c;
+	}
+};
+
 // FP32 Poisson draw on the keyed stream of the FP64 form (same counters/words).
 // The Philox blocks are computed by the warp's calling lanes together: when a
 // lane of the warp needs the inversion words of its column or the first PTRS
 // pair, every calling lane computes its own (same counters, so the same
 // values), instead of the warp issuing the block once for the inversion lanes
 // and again for the PTRS lanes.
-__device__ __forceinline__ int32_t poisson_fp32(float mean, uint32_t k0, uint32_t k1, uint32_t col, uint32_t tr,
-                                                uint32_t sett, uint32_t stream, U4 &inv, uint32_t &inv_call,
-                                                const float *rcp, const float *lnfact, uint32_t limit)
+template <typename Key>
+__device__ __forceinline__ int32_t poisson_fp32(float mean, const Key &key, uint32_t col, uint32_t tr, uint32_t sett,
+                                                uint32_t stream, U4 &inv, uint32_t &inv_call, const float *rcp,
+                                                const float *lnfact, uint32_t limit)
 {
 	const unsigned act = __activemask();
 	const bool big = mean >= 10.f;
 	const uint32_t call = tr >> 2;
 	if (__any_sync(act, !big && inv_call != call)) {
-		inv = philox10(U4{col, sett, stream, (PURPOSE_INV << 24) | call}, k0, k1);
+		inv = key(U4{col, sett, stream, (PURPOSE_INV << 24) | call});
 		inv_call = call;
 	}
 	U4 r0{0, 0, 0, 0};
-	if (__any_sync(act, big)) r0 = philox10(U4{col, sett, stream, (PURPOSE_PTRS << 24) | (tr << 16)}, k0, k1);
+	if (__any_sync(act, big)) r0 = key(U4{col, sett, stream, (PURPOSE_PTRS << 24) | (tr << 16)});
 	if (!big) {
 		// sequential search of the FP32 CDF: the smallest k with u <= F(k), or the k at
 		// which adding p(k) no longer changes F (the FP32 tail is exhausted), at most 63.
@@ -164,7 +187,7 @@ __device__ __forceinline__ int32_t poisson_fp32(float mean, uint32_t k0, uint32_
 	const float log_invalpha = __logf(invalpha);
 	const float two_a = 2.0f * a;
 	for (uint32_t it = 0; it < limit; it++) {
-		const U4 r = it == 0 ? r0 : philox10(U4{col, sett, stream, (PURPOSE_PTRS << 24) | (tr << 16) | it}, k0, k1);
+		const U4 r = it == 0 ? r0 : key(U4{col, sett, stream, (PURPOSE_PTRS << 24) | (tr << 16) | it});
 		const float U = u01_f(r.x) - 0.5f;
 		const float V = u01_f(r.y);
 		const float us = 0.5f - fabsf(U);
@@ -221,11 +244,6 @@ __device__ float obs_lp_fast(float vf, int o, const ModelDev &m)
 //    of matrix entries loads as one float2, eight sources in flight per lane
 //    (four in the 320-thread layouts).
 // The quad's partial sums are combined with two butterfly shuffles.
-// From 128 areas four targets per quad instead of two (640 threads, up to 12 ages: beyond, the
-// sums do not fit the registers): half the shared-memory reads per product, which bound the
-// other form (350 areas x 10 ages: 80,000 cycles per step before, 48,000 now).
-constexpr int kFoi4Areas = 128;
-
 template <int NT, int MG>
 __device__ __forceinline__ void foi(const ModelDev &m, const float *Ms, int lda, const float *Icnt, float *Imap, int tid)
 {
@@ -266,9 +284,11 @@ __device__ __forceinline__ void foi(const ModelDev &m, const float *Ms, int lda,
 					for (int q = 0; q < MG / 4; q++) Yt[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
 				}
 			}
-		} else if (NT >= 640 && MG <= 12 && A >= kFoi4Areas) {
-			// four targets per quad: a source's counts, read from shared memory, serve twice the
-			// products, and the next four sources' entries are in flight while these are used
+		} else if (NT >= 640 && MG <= 12 && A > NT / 2) {
+			// four targets per quad where two would need a second pass of the CTA: a source's
+			// counts, read from shared memory, serve twice the products, and the next four sources'
+			// entries are in flight while these are used (350 areas x 10 ages: 80,000 cycles per
+			// step with two targets, 48,000 now; beyond 12 ages the sums do not fit the registers)
 			constexpr int kU = 4;
 			const int nq = (A + 3) / 4;
 			for (int q0 = 0; q0 < nq; q0 += NT / 4) {
@@ -484,72 +504,85 @@ struct Tabs {
 // per (strain, area), the age-mixing matrix and the geographic spline
 // (src/state.cc:403-423, 547-553).  The loads for step sett are issued by
 // slice_load early in the previous step's draw phase and stored by slice_store
-// after it.  RAW: what is loaded is combined when it is stored, so that nothing
-// waits for the loads before the draws (small models, whose steps are bound by
-// latency: 1400 cycles of a 7900-cycle step); otherwise it is combined at once,
-// in fewer registers.
+// after it.
 struct SliceRegs {
-	float beta, af, ef, em, N, d;
+	float be, et, N, d;
 };
 
-// item i (strain, area) of a step's slices: beta, areafactor, external force of infection and its multiplier
-__device__ __forceinline__ void slice_item(const ModelDev &m, const Tabs &tb, const FastSmem &s, int sett, int i,
-                                           SliceRegs &r)
+// item i (strain, area) of a step's slices: beta * areafactor, external force of infection per capita
+__device__ __forceinline__ float2 slice_item(const ModelDev &m, const Tabs &tb, const FastSmem &s, int sett, int i)
 {
 	const int A = m.A, c = i % A;
-	r.beta = __ldg(tb.beta_rows + (size_t)s.brow[i] * m.S + sett);
-	r.af = __ldg(tb.areafactor + (size_t)(sett / m.div_per_time) * A + c);
-	r.ef = __ldg(tb.efoi_spline + (size_t)s.eref[i] * m.S + sett);
-	if (tb.efoi_mult) r.em = __ldg(tb.efoi_mult + ((size_t)sett * A + c) * m.NS + i / A);
-}
-
-__device__ __forceinline__ float2 slice_value(const ModelDev &m, const Tabs &tb, const SliceRegs &r)
-{
-	float et = r.ef * m.inv_popsize_f;
-	if (tb.efoi_mult) et *= r.em;
-	return make_float2(r.beta * r.af, et);
+	const float be = __ldg(tb.beta_rows + (size_t)s.brow[i] * m.S + sett) *
+	                 __ldg(tb.areafactor + (size_t)(sett / m.div_per_time) * A + c);
+	float et = __ldg(tb.efoi_spline + (size_t)s.eref[i] * m.S + sett) * m.inv_popsize_f;
+	if (tb.efoi_mult) et *= __ldg(tb.efoi_mult + ((size_t)sett * A + c) * m.NS + i / A);
+	return make_float2(be, et);
 }
 
 // the first NT items of each kind go through registers; items beyond (models
 // with more (strain, area) pairs or age pairs than threads) are loaded when stored
-template <int NT, bool RAW = false>
+template <int NT>
 __device__ __forceinline__ SliceRegs slice_load(const ModelDev &m, const Tabs &tb, const FastSmem &s, int sett, int tid)
 {
-	SliceRegs r{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+	SliceRegs r{0.f, 0.f, 0.f, 0.f};
 	if (tid < m.NS * m.A) {
-		slice_item(m, tb, s, sett, tid, r);
-		if constexpr (!RAW) {
-			const float2 v = slice_value(m, tb, r);
-			r.beta = v.x;
-			r.ef = v.y;
-		}
+		const float2 v = slice_item(m, tb, s, sett, tid);
+		r.be = v.x;
+		r.et = v.y;
 	}
 	if (tid < m.G * m.G) r.N = __ldg(tb.Ntime + (size_t)sett * m.G * m.G + tid);
 	if (tid == 0) r.d = __ldg(tb.geo + sett);
 	return r;
 }
 
-template <int NT, bool RAW = false>
+template <int NT>
 __device__ __forceinline__ void slice_store(const ModelDev &m, const Tabs &tb, FastSmem &s, const SliceRegs &r, int buf,
                                             int sett, int tid)
 {
 	float *be = buf ? s.be1 : s.be0, *et = buf ? s.et1 : s.et0, *N = buf ? s.N1 : s.N0;
 	const int NSA = m.NS * m.A, GG = m.G * m.G;
-	if (tid < NSA) {
-		const float2 v = RAW ? slice_value(m, tb, r) : make_float2(r.beta, r.ef);
-		be[tid] = v.x;
-		et[tid] = v.y;
-	}
+	if (tid < NSA) { be[tid] = r.be; et[tid] = r.et; }
 	if (tid < GG) N[tid] = r.N;
 	if (tid == 0) s.dgeo[buf] = r.d;
 	for (int i = tid + NT; i < NSA; i += NT) {
-		SliceRegs q;
-		slice_item(m, tb, s, sett, i, q);
-		const float2 v = slice_value(m, tb, q);
+		const float2 v = slice_item(m, tb, s, sett, i);
 		be[i] = v.x;
 		et[i] = v.y;
 	}
 	for (int i = tid + NT; i < GG; i += NT) N[i] = __ldg(tb.Ntime + (size_t)sett * GG + i);
+}
+
+// The same for small models, whose steps are bound by latency: what is loaded is combined
+// when it is stored, so that nothing waits for the loads before the draws (1400 cycles of a
+// 7900-cycle step).
+struct SliceRaw {
+	float beta, af, ef, em, N, d;
+};
+
+template <int NT>
+__device__ __forceinline__ SliceRaw slice_load_raw(const ModelDev &m, const Tabs &tb, const FastSmem &s, int sett, int tid)
+{
+	SliceRaw r{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+	if (tid < m.NS * m.A) {
+		const int A = m.A, c = tid % A;
+		r.beta = __ldg(tb.beta_rows + (size_t)s.brow[tid] * m.S + sett);
+		r.af = __ldg(tb.areafactor + (size_t)(sett / m.div_per_time) * A + c);
+		r.ef = __ldg(tb.efoi_spline + (size_t)s.eref[tid] * m.S + sett);
+		if (tb.efoi_mult) r.em = __ldg(tb.efoi_mult + ((size_t)sett * A + c) * m.NS + tid / A);
+	}
+	if (tid < m.G * m.G) r.N = __ldg(tb.Ntime + (size_t)sett * m.G * m.G + tid);
+	if (tid == 0) r.d = __ldg(tb.geo + sett);
+	return r;
+}
+
+template <int NT>
+__device__ __forceinline__ void slice_store_raw(const ModelDev &m, const Tabs &tb, FastSmem &s, const SliceRaw &r, int buf,
+                                                int sett, int tid)
+{
+	float et = r.ef * m.inv_popsize_f;
+	if (tb.efoi_mult) et *= r.em;
+	slice_store<NT>(m, tb, s, SliceRegs{r.beta * r.af, et, r.N, r.d}, buf, sett, tid);
 }
 
 // an observation's accumulator v plus its cells of the step, weighted
@@ -1000,7 +1033,7 @@ __device__ __forceinline__ int pd_steps(const ModelDev &m, const BatchDev &b, co
 	int sb = 0, a0 = b.step_ptr[0], a1 = b.step_ptr[1];
 	for (int sett = b.ti; sett < b.tf; sett++) {
 		int32_t *pc = cur ? s.pop1 : s.pop0, *pn = cur ? s.pop0 : s.pop1;
-		const SliceRegs nxt = sett + 1 < b.tf ? slice_load<NT, true>(m, tb, s, sett + 1, tid) : SliceRegs{};
+		const SliceRaw nxt = sett + 1 < b.tf ? slice_load_raw<NT>(m, tb, s, sett + 1, tid) : SliceRaw{};
 		const int a2 = b.step_ptr[min(sett + 2 - b.ti, nsteps)];
 		int4 t0 = make_int4(0, 0, 0, 0), t1 = make_int4(0, 0, 0, 0);
 		const bool first = a0 + otid < a1;
@@ -1059,7 +1092,7 @@ __device__ __forceinline__ int pd_steps(const ModelDev &m, const BatchDev &b, co
 			if (mean > 0.f) {
 				if (mean > 1.0e9f) atomicCAS(status, 0, BEEP_COUNT_OVERFLOW);
 				else {
-					n = poisson_fp32(mean, k0, k1, (uint32_t)q.col, (uint32_t)q.tr, (uint32_t)sett, stream, inv, inv_call,
+					n = poisson_fp32(mean, KeyRegs{k0, k1}, (uint32_t)q.col, (uint32_t)q.tr, (uint32_t)sett, stream, inv, inv_call,
 					                 s.rcp, s.lnfact, lim);
 					if (n < 0) { atomicCAS(status, 0, BEEP_TIMEOUT); n = 0; }
 				}
@@ -1096,7 +1129,7 @@ __device__ __forceinline__ int pd_steps(const ModelDev &m, const BatchDev &b, co
 			if (m.dp_age_unique) Ic_nxt[(st * A + c) * MG + a] = iv;
 			else atomicAdd(Ic_nxt + (st * A + c) * MG + a, iv);
 		}
-		if (sett + 1 < b.tf) slice_store<NT, true>(m, tb, s, nxt, sb ^ 1, sett + 1, tid);
+		if (sett + 1 < b.tf) slice_store_raw<NT>(m, tb, s, nxt, sb ^ 1, sett + 1, tid);
 		__syncthreads();
 		// ---- outputs, observations, the next force of infection
 		if (b.pop_traj)
@@ -1320,7 +1353,7 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 	if constexpr (PD) red_at = pd_steps<NT, MG>(m, b, tb, s, p, stream, k0, k1, lda, Lsum, Lcmp, cur);
 	for (int sett = b.ti; sett < b.tf && tc_ok && !PD; sett++) {
 		int32_t *pc = cur ? s.pop1 : s.pop0, *pn = cur ? s.pop0 : s.pop1;
-		const SliceRegs nxt = sett + 1 < b.tf ? slice_load<NT>(m, tb, s, sett + 1, tid) : SliceRegs{};
+		const SliceRegs nxt = sett + 1 < b.tf ? slice_load<NT>(m, tb, s, sett + 1, tid) : SliceRegs{0.f, 0.f, 0.f, 0.f};
 		const float *be = sb ? s.be1 : s.be0, *et = sb ? s.et1 : s.et0, *Nm = sb ? s.N1 : s.N0;
 		const float *Ic_cur = cur ? s.Ic1 : s.Ic0;
 		float *Ic_nxt = cur ? s.Ic0 : s.Ic1;
@@ -1425,13 +1458,13 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 						if (mean > 0.f) {
 							if (mean > 1.0e9f) atomicCAS(status, 0, BEEP_COUNT_OVERFLOW);
 							else if (b.simu_all || (b.simu && b.simu[((size_t)p * m.S + sett) * A + c])) {
-								n = poisson_fp32(mean, k0, k1, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, inv,
+								n = poisson_fp32(mean, KeyRegs{k0, k1}, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, inv,
 								                 inv_call, s.rcp, s.lnfact, lim);
 							} else {                       // coupled to the current state (src/mbp.cc:293-305)
 								const int32_t ni = b.ch_tn[ci];
 								const float ri = b.ch_mean_f[ci];
 								if (mean > ri) {
-									n = poisson_fp32(mean - ri, k0, k1, (uint32_t)col, (uint32_t)tr, (uint32_t)sett,
+									n = poisson_fp32(mean - ri, KeyRegs{k0, k1}, (uint32_t)col, (uint32_t)tr, (uint32_t)sett,
 									                 stream, inv, inv_call, s.rcp, s.lnfact, lim);
 									if (n >= 0) n += ni;
 								} else if (mean == ri) n = ni;
@@ -1447,7 +1480,7 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 				if (mean > 0.f) {
 					if (mean > 1.0e9f) atomicCAS(status, 0, BEEP_COUNT_OVERFLOW);
 					else {
-						n = poisson_fp32(mean, k0, k1, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, inv, inv_call,
+						n = poisson_fp32(mean, KeyRegs{k0, k1}, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, inv, inv_call,
 						                 s.rcp, s.lnfact, lim);
 						if (n < 0) { atomicCAS(status, 0, BEEP_TIMEOUT); n = 0; }
 					}
@@ -1549,8 +1582,9 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 	}
 	if (b.L) {
 		__syncthreads();
-		s.red[red_at] = Lsum;
-		s.red[NT + red_at] = Lcmp;
+		const int at = PD ? red_at : tid;
+		s.red[at] = Lsum;
+		s.red[NT + at] = Lcmp;
 		__syncthreads();
 		if (tid < 32) {
 			double S = 0.0;
