@@ -23,7 +23,9 @@
 //                 bounded by 1.5e-6 (2e-6) of it plus 2e-6 for the fraction of the mean.
 //   vr            2e-6 absolute
 //   acceptance    1e-4 + 2e-6 |d| (4e-6 |d|) + 1e-6 |rhs|, d = mean - (k+1) or k - m, with
-//                 the density written without cancellation (as the fast form's).
+//                 the density written without cancellation (as the fast form's), its log Gamma
+//                 remainders within 5e-6 (stirling_rem_f32).
+// tests/test_filtered_draws.py puts 1e6 draws at the places where a decision turns.
 // Redone draws: 1 in 11,000 at means of 1 to 10, 1 in 3,000 at 10 to 1000, 1 in 1,000 up to 1e5,
 // 1 in 130 up to 1e7.  Per draw and SM: 26 -> 1.1 ns at mean 1, 255 -> 5.4 ns at 20, 137 -> 11 ns
 // at 1e5 (2.5e8 draws over means 1e-6 to 1e9, and as many binomials, equal to the FP64 ones).
@@ -163,10 +165,13 @@ __device__ __forceinline__ int32_t poisson_filtered(double mean, uint32_t k0, ui
 	return poisson_fp64(mean, k0, k1, col, tr, sett, stream, limit);   // an uncertain comparison (or `limit` rejections)
 }
 
-__device__ __forceinline__ float stirling_rem_f32(float z)   // log Gamma(z) - ((z - 1/2) log z - z + log(2 pi)/2)
+// log Gamma(z) - ((z - 1/2) log z - z + log(2 pi)/2) of an integer z: three terms of the series, off
+// by less than the first one omitted, 1 / (1680 z^7) <= 5e-6, from z = 2 on; at z = 1 (a candidate of
+// 0 or of n) they would be 2.9e-4 off, so the value itself stands there, 1 - log(2 pi)/2
+__device__ __forceinline__ float stirling_rem_f32(float z)
 {
 	const float iz = __fdividef(1.f, z), iz2 = iz * iz;
-	return iz * (0.083333333f - iz2 * (0.0027777778f - iz2 * 0.00079365079f));
+	return z < 1.5f ? 0.081061467f : iz * (0.083333333f - iz2 * (0.0027777778f - iz2 * 0.00079365079f));
 }
 
 // binomial_fp64's draw
