@@ -588,6 +588,16 @@ beep_status check_batch(const beep_model *m, const beep_sim_batch *b, bool devic
 	return BEEP_OK;
 }
 
+// External-force tables a particle's CTA stages in shared memory: those of the parameter sets
+// where all have as many and they are at most 1024 values, else none (read from L2).
+int32_t efoi_tables_to_stage(const beep_model *m, const beep_sim_batch *b)
+{
+	const int32_t n = b->groups[0].nefoi;
+	for (int g = 1; g < b->ngroup; g++)
+		if (b->groups[g].nefoi != n) return 0;
+	return n > 0 && (long long)n * m->G <= 1024 ? n : 0;
+}
+
 // Packs the caller's current host arrays into the pinned staging buffer.
 beep_status stage_inputs(beep_batch *q)
 {
@@ -672,6 +682,9 @@ beep_status stage_inputs(beep_batch *q)
 	bd.step_obs = (const int32_t *)(di + o_sobs);
 	bd.fpool32 = fast ? (const float *)(di + o_f32) : nullptr;
 	bd.tasks = (const int4 *)(di + o_tasks);
+	// the shared-memory layout holds the tables the batch was created with: tables of another
+	// number are read from L2
+	if (fast) bd.nefoi_stage = efoi_tables_to_stage(m, b) == q->nefoi_layout ? q->nefoi_layout : 0;
 	return BEEP_OK;
 }
 
@@ -777,12 +790,7 @@ beep_status beep::batch_create_internal(beep_model *m, const beep_sim_batch *b, 
 				t[4] = fbits; t[5] = m->obs_spline[o]; t[6] = c0; t[7] = run;
 			}
 		const size_t limit = 227 * 1024;
-		int nefoi = 1 << 30;
-		for (int g = 0; g < b->ngroup; g++) nefoi = std::min(nefoi, (int)b->groups[g].nefoi);
-		if (b->ngroup > 1)
-			for (int g = 1; g < b->ngroup; g++)
-				if (b->groups[g].nefoi != b->groups[0].nefoi) nefoi = 0;
-		q->bd.nefoi_stage = nefoi * m->G <= 1024 ? nefoi : 0;
+		q->nefoi_layout = q->bd.nefoi_stage = efoi_tables_to_stage(m, b);
 		// counts of unobserved transitions are not stored unless a trajectory is requested; one
 		// population buffer suffices when no observation reads populations and strains do not mix
 		q->bd.tn_full = traj ? 1 : 0;
@@ -1123,7 +1131,10 @@ beep_status beep_batch_run_graph(beep_batch *q)
 	beep_status st = beep_batch_stage(q);
 	if (st != BEEP_OK) return st;
 	cudaStream_t s = q->m->stream;
-	if (q->graph_exec && q->graph_in_size != q->in_size) {   // the staged inputs changed size: capture again
+	q->bd.sampler_limit = option_sampler_limit();
+	// the launches' arguments are part of the graph: capture again where staging changed one (the
+	// inputs' sizes and places, the external-force tables staged) or the option did
+	if (q->graph_exec && (q->graph_in_size != q->in_size || memcmp(&q->graph_bd, &q->bd, sizeof(BatchDev)) != 0)) {
 		cudaGraphExecDestroy(q->graph_exec);
 		cudaGraphDestroy(q->graph);
 		q->graph_exec = nullptr;
@@ -1149,6 +1160,7 @@ beep_status beep_batch_run_graph(beep_batch *q)
 		}
 		q->graph = g;
 		q->graph_in_size = q->in_size;
+		memcpy(&q->graph_bd, &q->bd, sizeof(BatchDev));
 	}
 	CUDA_TRY(cudaGraphLaunch(q->graph_exec, s));
 	CUDA_TRY(cudaStreamSynchronize(s));

@@ -219,6 +219,8 @@ struct beep_batch {
 	cudaGraph_t graph = nullptr;
 	cudaGraphExec_t graph_exec = nullptr;
 	size_t graph_in_size = 0;
+	beep::BatchDev graph_bd{};   // the arguments it was captured with
+	int32_t nefoi_layout = 0;    // external-force tables the fast form's shared-memory layout holds
 };
 
 
