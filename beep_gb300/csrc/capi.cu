@@ -901,12 +901,18 @@ beep_status beep::batch_create_internal(beep_model *m, const beep_sim_batch *b, 
 		// sequential chain of draws per thread (the particle filter's sections are this case)
 		const int popt = option_parallel_draws();
 		const int nt_run = q->bd.nt > 0 ? q->bd.nt : fast_pick_threads(m->dev);
-		q->bd.pd = !wide && !q->bd.foi_tc && !q->bd.batched && fast_pd_fits(m->dev, nt_run) && popt != 1 &&
+		// (where their array of population changes fits beside the layout chosen above)
+		auto pd_fits = [&](int nt) {
+			return fast_pd_fits(m->dev, nt) &&
+			       fast_smem_bytes(m->dev, nslots, q->bd.m_in_smem != 0, q->bd.nefoi_stage, q->state_global, tnrows, ps,
+			                       false, nt, 0, true) <= limit;
+		};
+		q->bd.pd = !wide && !q->bd.foi_tc && !q->bd.batched && popt != 1 && pd_fits(nt_run) &&
 		           (popt == 2 || (long long)P <= 4LL * std::max(1, m->sms)) ? 1 : 0;
 		// one pass of 256 threads over the draws instead of two of 128, where the batch
 		// leaves room for the larger CTAs (two per SM)
 		if (q->bd.pd && popt != 2 && nt_run == 128 && (long long)m->T * m->A * m->DP > 128 &&
-		    (long long)P <= 2LL * std::max(1, m->sms))
+		    (long long)P <= 2LL * std::max(1, m->sms) && pd_fits(256))
 			q->bd.nt = 256;
 	}
 	auto bail = [&](beep_status s) { beep_batch_destroy(q); return s; };
