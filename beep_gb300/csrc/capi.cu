@@ -445,7 +445,7 @@ beep_status beep_model_destroy(beep_model *m)
 	if (m->stream) cudaStreamSynchronize(m->stream);
 	for (beep_batch *q : m->pf.q) beep_batch_destroy(q);
 	m->pf.q.clear();
-	m->pf.work.release();
+	m->pf.work.release(m->pool.get());
 	m->model_mem.release(m->pool.get());
 	if (m->stream) cudaStreamDestroy(m->stream);
 	delete m;

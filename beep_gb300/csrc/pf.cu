@@ -198,7 +198,8 @@ extern "C" BEEP_API beep_status beep_pf_loglik(beep_model *m, const beep_pf_requ
 	             o_ws = L.add(8 * (size_t)N), o_sel = L.add(4 * (size_t)N), o_fi = L.add(4 * (size_t)N),
 	             o_ex = L.add(4 * (size_t)N), o_ob = L.add(8 * (size_t)ns), o_anc = L.add(4 * (size_t)ns * N),
 	             o_pst = L.add(4 * ((size_t)ns * N + 1));
-	cudaError_t e = pc.work.reserve(L.size);
+	if (pc.work.cap < L.size) pc.work.release(m->pool.get());   // (nothing is in flight between calls)
+	cudaError_t e = pc.work.reserve(L.size, m->pool.get());
 	if (e != cudaSuccess) { drop_cache(); return fail(BEEP_OOM, std::string("particle filter buffers: ") + cudaGetErrorString(e)); }
 	char *d = (char *)pc.work.ptr;
 	int32_t *pops[2] = {(int32_t *)(d + o_pa), (int32_t *)(d + o_pb)};   // the sections' final populations, in turn
