@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <memory>
@@ -30,14 +31,26 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Device and pinned buffers of destroyed batches and models, kept for the next ones: an
 // allocation, and above all a release, of either kind costs 0.1 to 1 ms and waits for the
-// whole device.  A pool belongs to a model (its batches come and go, one per beep_simulate)
+// whole device.  What pools keep never makes an allocation fail: one that does is tried again
+// with every pool of the process emptied (driver_alloc).  A pool belongs to a model (its batches come and go, one per beep_simulate)
 // or to a server (models and batches per request); it keeps at most `limit` bytes of each kind
 // and goes with its last owner.  Buffers are given back only when no work that uses them is
 // left in flight.  Safe from several threads.
 class BufPool {
 public:
-	explicit BufPool(size_t limit) : limit_(limit) {}
-	~BufPool() { trim(0); }
+	explicit BufPool(size_t limit) : limit_(limit)
+	{
+		std::lock_guard<std::mutex> lk(all().mu);
+		all().pools.push_back(this);
+	}
+	~BufPool()
+	{
+		{
+			std::lock_guard<std::mutex> lk(all().mu);
+			all().pools.erase(std::find(all().pools.begin(), all().pools.end(), this));
+		}
+		trim(0);
+	}
 	BufPool(const BufPool &) = delete;
 	BufPool &operator=(const BufPool &) = delete;
 	cudaError_t take(bool host, size_t n, void **ptr, size_t *cap)
@@ -60,13 +73,24 @@ public:
 				return cudaSuccess;
 			}
 		}
+		const cudaError_t e = driver_alloc(host, n, ptr);
+		*cap = e == cudaSuccess ? n : 0;
+		return e;
+	}
+	// Memory from the driver; where there is none left, every pool gives its spare buffers back
+	// first.
+	static cudaError_t driver_alloc(bool host, size_t n, void **ptr)
+	{
 		cudaError_t e = host ? cudaMallocHost(ptr, n) : cudaMalloc(ptr, n);
 		if (e == cudaErrorMemoryAllocation) {
 			cudaGetLastError();
-			trim(0);
+			{
+				std::lock_guard<std::mutex> lk(all().mu);
+				for (BufPool *p : all().pools) p->trim(0);
+			}
 			e = host ? cudaMallocHost(ptr, n) : cudaMalloc(ptr, n);
+			if (e == cudaErrorMemoryAllocation) cudaGetLastError();   // (the caller's to report, not a later launch's)
 		}
-		*cap = e == cudaSuccess ? n : 0;
 		if (e != cudaSuccess) *ptr = nullptr;
 		return e;
 	}
@@ -105,6 +129,16 @@ public:
 	}
 
 private:
+	// the pools of the process (never destroyed: a pool may outlive the library's statics)
+	struct All {
+		std::mutex mu;
+		std::vector<BufPool *> pools;
+	};
+	static All &all()
+	{
+		static All *a = new All;
+		return *a;
+	}
 	struct Buf {
 		void *ptr;
 		size_t cap;
@@ -130,9 +164,8 @@ struct GrowBuf {
 		if (n <= cap) return cudaSuccess;
 		release();
 		if (pool) return pool->take(HOST, n, &ptr, &cap);
-		const cudaError_t e = HOST ? cudaMallocHost(&ptr, n) : cudaMalloc(&ptr, n);
+		const cudaError_t e = BufPool::driver_alloc(HOST, n, &ptr);
 		if (e == cudaSuccess) cap = n;
-		else ptr = nullptr;
 		return e;
 	}
 	void release(BufPool *pool = nullptr)

@@ -200,7 +200,12 @@ BEEP_API const char *beep_last_error(void);
 BEEP_API beep_status beep_device_init(int32_t device);
 
 /* Model lifetime (replaces constructing Data/Model/ObservationModel for the
- * hot path: src/main.cc:148-160). */
+ * hot path: src/main.cc:148-160).
+ * A model keeps the buffers of destroyed batches (each beep_simulate makes one)
+ * and of its filters for the next: at most 256 MiB of device memory and as much
+ * pinned host memory, given back when the model is destroyed or when an
+ * allocation of this library, for any model or server of the process, finds no
+ * memory left.  Allocations outside the library cannot reclaim them. */
 BEEP_API beep_status beep_model_create(const beep_model_desc *desc, beep_model **out);
 BEEP_API beep_status beep_model_destroy(beep_model *model);
 
@@ -513,7 +518,9 @@ typedef struct beep_request_stats {
 
 typedef struct beep_server beep_server;
 /* hbm_budget_bytes: device memory the server's requests may hold at once
- * (a request larger than the budget runs alone). */
+ * (a request larger than the budget runs alone).  Within it the server keeps
+ * finished requests' buffers for later ones: down to 256 MiB once nothing runs
+ * or waits, and none of them when the oldest request waits for room. */
 BEEP_API beep_status beep_server_create(int32_t device, int64_t hbm_budget_bytes, int32_t max_inflight,
                                         beep_server **out);
 /* Finishes every submitted request, then releases the server. */
