@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -282,7 +283,11 @@ beep_status batch_launch_kernels(beep_batch *q);
 // copy into the caller's arrays.
 beep_status batch_download_enqueue(beep_batch *q);
 beep_status batch_download_finish(beep_batch *q);
-// Device bytes held by a model / a batch.
+// beep_pf_loglik; ready (may be null) is called once its device buffers are in place, before
+// the sections are launched.
+beep_status pf_loglik(beep_model *m, const beep_pf_request *r, const std::function<void()> &ready);
+// Device bytes held by a model / a batch / a model's filter.
 size_t model_device_bytes(const beep_model *m);
 size_t batch_device_bytes(const beep_batch *q);
+size_t pf_device_bytes(const beep_model *m);
 }  // namespace beep

@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kBootThreads) pf_bootstrap(const double *L, in
 
 using namespace beep;
 
-extern "C" BEEP_API beep_status beep_pf_loglik(beep_model *m, const beep_pf_request *r)
+beep_status beep::pf_loglik(beep_model *m, const beep_pf_request *r, const std::function<void()> &ready)
 {
 	if (!m || !r || !r->tables) return fail(BEEP_BAD_INPUT, "null argument");
 	const int N = r->nparticle, ns = r->nsection;
@@ -201,6 +201,7 @@ extern "C" BEEP_API beep_status beep_pf_loglik(beep_model *m, const beep_pf_requ
 	if (pc.work.cap < L.size) pc.work.release(m->pool.get());   // (nothing is in flight between calls)
 	cudaError_t e = pc.work.reserve(L.size, m->pool.get());
 	if (e != cudaSuccess) { drop_cache(); return fail(BEEP_OOM, std::string("particle filter buffers: ") + cudaGetErrorString(e)); }
+	if (ready) ready();
 	char *d = (char *)pc.work.ptr;
 	int32_t *pops[2] = {(int32_t *)(d + o_pa), (int32_t *)(d + o_pb)};   // the sections' final populations, in turn
 	double *Lall = (double *)(d + o_L), *obsec = (double *)(d + o_ob);
@@ -288,3 +289,12 @@ extern "C" BEEP_API beep_status beep_pf_loglik(beep_model *m, const beep_pf_requ
 	if (r->loglik_section_out) memcpy(r->loglik_section_out, ob.data(), 8 * (size_t)ns);
 	return BEEP_OK;
 }
+
+size_t beep::pf_device_bytes(const beep_model *m)
+{
+	size_t n = m->pf.work.cap;
+	for (const beep_batch *q : m->pf.q) n += batch_device_bytes(q);
+	return n;
+}
+
+extern "C" BEEP_API beep_status beep_pf_loglik(beep_model *m, const beep_pf_request *r) { return pf_loglik(m, r, nullptr); }

@@ -141,7 +141,15 @@ size_t estimate_pf_bytes(const beep_model_desc &d, const beep_pf_request &r)
 	b.L_out = &L;
 	const size_t N = r.nparticle, popsz = (size_t)d.narea * d.ncomp * d.ndemocatpos;
 	const size_t tnsz = (size_t)d.narea * d.ntrans * d.ndemocatpos;
-	return 2 * estimate_bytes(d, b) + N * ((d.ndemocat_change > 0 ? 16 : 8) * popsz + 64 + 12 * (size_t)r.nsection) +
+	// each section's batch has its particles' work arrays (plain form) and the tables
+	const size_t agsz = (size_t)d.nstrain * d.narea * d.nage, pe = d.ndemocat_change > 0 ? 8 : 4;
+	const beep_param_tables &t = *r.tables;
+	const size_t S = d.ndivision, value = r.form == BEEP_FORM_FAST ? 4 : 8;
+	const size_t section = (r.form == BEEP_FORM_FAST ? 0 : N * (2 * pe * popsz + 4 * tnsz + 32 * agsz)) + 16384 +
+	                       value * (S * ((size_t)t.nbeta_row + t.nefoi + t.nobs_spline + (size_t)d.nage * d.nage + 1) +
+	                                (size_t)d.period * d.narea + (size_t)d.ntrans * d.ndemocatpos);
+	return 2 * estimate_bytes(d, b) + section * (size_t)r.nsection +
+	       N * ((d.ndemocat_change > 0 ? 16 : 8) * popsz + 64 + 12 * (size_t)r.nsection) +
 	       (r.lineage_transnum_out ? 4 * tnsz * (size_t)d.ndivision * N : 0);
 }
 
@@ -202,7 +210,15 @@ void run_pf_request(beep_server *s, Req *r)
 		cudaEventCreate(&r->ev_start);
 		cudaEventCreate(&r->ev_end);
 		cudaEventRecord(r->ev_start, r->m->stream);
-		st = beep_pf_loglik(r->m, &r->pf);
+		// charged with its estimate until its buffers are in place, then with what they take (a spare
+		// buffer of the pool may be larger than asked for)
+		st = pf_loglik(r->m, &r->pf, [s, r] {
+			const size_t bytes = model_device_bytes(r->m) + pf_device_bytes(r->m);
+			std::lock_guard<std::mutex> lk(s->mu);
+			s->used = s->used - r->bytes + bytes;
+			r->bytes = bytes;
+			s->held = s->pool->device_bytes();
+		});
 		cudaEventRecord(r->ev_end, r->m->stream);
 		cudaEventSynchronize(r->ev_end);
 		float a = 0, b = 0;
@@ -419,7 +435,7 @@ void worker_main(beep_server *s)
 			lk.unlock();
 			start_request(s, r);
 			lk.lock();
-			s->used = s->used - r->est + r->bytes;
+			if (r->kind != BEEP_REQ_PF_LIKELIHOOD) s->used = s->used - r->est + r->bytes;   // (a filter's thread does it)
 			s->held = s->pool->device_bytes();
 			s->running.push_back(r);   // a failed start retires at the next pass
 		}

@@ -49,3 +49,19 @@ def test_a_finished_filter_does_not_hold_up_other_requests():
     assert srv.stats(k)["state"] == 1                     # the long one still runs
     srv.wait(k, 120.0)
     srv.close()
+
+
+def test_a_filter_is_charged_what_it_holds():
+    m, t = model(30, 4, 40, 2)
+    N, S = 400, m.ndivision
+    sections = [(k, k + 2) for k in range(0, S, 2)]
+    srv = capi.Server(8 << 30, 2)
+    big = capi.Batch(m, [t], 3000, 1, want_pop=True)       # its buffers go to the pool: larger than the filter's
+    k = srv.submit(m, big, capi.REQ_LIKELIHOOD)
+    srv.wait(k, 60.0)
+    k = srv.submit_pf(m, t, N, 5, 1, 0.5, sections)
+    srv.wait(k, 60.0)
+    ncol = m.narea * m.ndemocatpos
+    per = 4 * (2 * m.ncomp + m.ntrans) * ncol + 8 * 4 * m.nstrain * m.narea * m.nage   # a particle's work in a section
+    assert srv.stats(k)["device_bytes"] >= len(sections) * N * per
+    srv.close()
