@@ -18,6 +18,7 @@ struct ModelDev {
 	int32_t A, G, DP, NS, DPS, C, T, S, period, div_per_time, nobs;
 	int32_t infection_trans;
 	double dt, popsize;
+	double efoi_zero;                    // 0 / popsize: 0, or NaN where the population size is no divisor
 	const int32_t *trans_from, *trans_to, *dp_age;
 	const double *M_diag, *M_factor;
 	const int32_t *csc_ptr, *csc_src;    // [A+1], [nnz]

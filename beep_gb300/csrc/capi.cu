@@ -392,6 +392,7 @@ beep_status beep::model_create_internal(const beep_model_desc *d, std::shared_pt
 	md.A = A; md.G = G; md.DP = DP; md.NS = NS; md.DPS = DPS; md.C = C; md.T = T; md.S = S;
 	md.period = d->period; md.div_per_time = d->division_per_time; md.nobs = nobs;
 	md.infection_trans = d->infection_trans; md.dt = d->dt; md.popsize = d->popsize;
+	md.efoi_zero = 0.0 / d->popsize;
 	md.trans_from = (const int32_t *)(base + o_tf); md.trans_to = (const int32_t *)(base + o_tt);
 	md.dp_age = (const int32_t *)(base + o_age); md.M_diag = (const double *)(base + o_diag);
 	md.M_factor = (const double *)(base + o_fac); md.csc_ptr = (const int32_t *)(base + o_cp);

@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 	};
 	auto slice_value = [&](double be, double af, double et, double em, double &b_out, double &e_out) {
 		b_out = be * af;
-		if (!is_zero(et)) et = et / m.popsize;
+		et = is_zero(et) ? m.efoi_zero : et / m.popsize;
 		if (efoi_mult) et *= em;
 		e_out = et;
 	};
