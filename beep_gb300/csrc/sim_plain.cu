@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 						n0 = item == tid ? first_n : b.ch_tn[ci];
 						ri = item == tid ? first_r : b.ch_mean[ci];
 						draw = mean - ri;
-						thin = mean < ri;
+						thin = !(mean >= ri);           // (a NaN current mean draws as the binomial of NaN: 0)
 					}
 					if (thin) n = binomial_filtered(mean / ri, n0, k0, k1, (uint32_t)col, (uint32_t)tr, (uint32_t)sett, stream, lim, ftab);
 					else {
