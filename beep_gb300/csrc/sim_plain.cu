@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 			if (tr == itr) {
 				const int st = dp / DPS, dpl = dp - st * DPS;
 				const PopT popu = pop_cur[((size_t)c * C + inf_from) * DP + dpl];
-				if (popu > 0) {
+				if (!(popu <= 0)) {                // (a NaN population's rate is NaN)
 					const int sc = st * A + c, a = age[dpl];
 					double nmi;
 					if (G == 1) nmi = X[sc];
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(kMaxThreads) sim_plain_kernel(const ModelDev m
 				}
 			} else {
 				const PopT popu = pop_cur[((size_t)c * C + from[tr]) * DP + dp];
-				if (popu > 0) mean = m.dt * (double)popu * rate[tr * DP + dp];
+				if (!(popu <= 0)) mean = m.dt * (double)popu * rate[tr * DP + dp];
 			}
 			if (tm_mult) mean *= tm_mult[(size_t)sett * tnsz + cell];   // prediction modifications
 			const bool bad = is_nan(mean);
