@@ -116,7 +116,8 @@ __device__ __forceinline__ int32_t search_cdf(float u, float p, float bound0, fl
 	return -2;
 }
 
-// poisson_fp64's draw (mean > 0, finite, at most 1e9)
+// poisson_fp64's draw (mean > 0).  Beyond 1e9, which only the difference from a negative current mean
+// reaches, by the FP64 function: the integer part is kept in 32 bits here.
 __device__ __forceinline__ int32_t poisson_filtered(double mean, uint32_t k0, uint32_t k1, uint32_t col, uint32_t tr,
                                                     uint32_t sett, uint32_t stream, uint32_t limit, const FilterTab &t)
 {
@@ -128,6 +129,7 @@ __device__ __forceinline__ int32_t poisson_filtered(double mean, uint32_t k0, ui
 		                             [mf](float p, int32_t) { return p * mf; });
 		return k >= 0 ? k : poisson_fp64(mean, k0, k1, col, tr, sett, stream, limit);
 	}
+	if (__double_as_longlong(mean) > __double_as_longlong(1e9)) return poisson_fp64(mean, k0, k1, col, tr, sett, stream, limit);
 	float frac;
 	const int32_t whole = split_pos(mean, frac);
 	const float b = fmaf(2.53f, __fsqrt_rn(mf), 0.931f);

@@ -137,6 +137,12 @@ int64_t boundary_trials(double par, int32_t n, const int32_t *want, int nwant, T
 	return o.len;
 }
 
+// the FP64 sampler's draws of the trials' words
+void fp64_host(Trial *t, int64_t len)
+{
+	for (int64_t k = 0; k < len; k++) t[k].fp64 = trial_fp64(t[k].par, t[k].n, t[k].x, t[k].y, 2);
+}
+
 // the filtered samplers' results on the host, the approximate operations off by `off`
 void filtered_host(const Trial *t, int64_t len, int off, int32_t *out)
 {

@@ -47,6 +47,8 @@ def host(tmp_path_factory):
     L.boundary_trials.argtypes = [C.c_double, C.c_int32, C.c_void_p, C.c_int, C.c_void_p, C.c_int64]
     L.filtered_host.argtypes = [C.c_void_p, C.c_int64, C.c_int, C.c_void_p]
     L.filtered_host.restype = None
+    L.fp64_host.argtypes = [C.c_void_p, C.c_int64]
+    L.fp64_host.restype = None
     return L, tmp
 
 
@@ -117,6 +119,21 @@ def test_a_binomial_draw_of_zero(host):
     got = np.empty(1, np.int32)
     L.filtered_host(t.ctypes.data, 1, 4, got.ctypes.data)
     assert got[0] == 0
+
+
+@pytest.mark.parametrize("mean", (0.999e9, 1.001e9, 2.147e9, 2.2e9, 5e9, 1e12, float("inf")))
+def test_means_around_and_beyond_32_bits(host, mean):
+    """The draws' words at random: the FP64 sampler's counts, whatever it makes of a mean beyond them."""
+    L, _ = host
+    rng = np.random.default_rng(5)
+    t = np.zeros(2000, TRIAL)
+    t["par"], t["n"] = mean, -1
+    t["x"], t["y"] = rng.integers(0, 1 << 32, (2, len(t)), dtype=np.uint32)
+    L.fp64_host(t.ctypes.data, len(t))
+    got = np.empty(len(t), np.int32)
+    for off in range(5):
+        L.filtered_host(t.ctypes.data, len(t), off, got.ctypes.data)
+        assert np.array_equal(t["fp64"], got), report(t, got)
 
 
 @pytest.mark.gpu
