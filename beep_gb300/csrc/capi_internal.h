@@ -56,9 +56,10 @@ public:
 	BufPool &operator=(const BufPool &) = delete;
 	cudaError_t take(bool host, size_t n, void **ptr, size_t *cap)
 	{
-		// sizes in steps of 1/8 of their power of two, so that batches of near sizes share buffers
+		// sizes in steps of 1/8 of their power of two, so that batches of near sizes share buffers;
+		// at most 2 MiB, the driver's own granularity, so that a batch fits where its bytes do
 		size_t step = 4096;
-		while (step * 16 < n) step *= 2;
+		while (step * 16 < n && step < (size_t)2 << 20) step *= 2;
 		n = align_up(n, step);
 		{
 			std::lock_guard<std::mutex> lk(mu_);

@@ -136,6 +136,25 @@ int a_pool_keeps_its_limit_and_trims_the_oldest()
 	return 0;
 }
 
+int large_buffers_take_what_they_ask_for()
+{
+	reset((size_t)270000 * kMB, (size_t)100000 * kMB);
+	{
+		BufPool a(256 * kMB), server((size_t)200000 * kMB);
+		for (BufPool *pool : {&a, &server})
+			for (size_t n : {(size_t)270000 * kMB, (size_t)131073 * kMB, (size_t)33 * kMB + 1, (size_t)5 * kMB + 7}) {
+				DevBuf x;
+				EXPECT(x.reserve(n, pool) == cudaSuccess && x.cap - n < 2 * kMB);
+				x.release();
+			}
+		HostBuf h;
+		EXPECT(h.reserve((size_t)100000 * kMB, &a) == cudaSuccess);
+		h.release();
+	}
+	EXPECT(drv.used[0] == 0 && drv.used[1] == 0 && drv.errors == 0);
+	return 0;
+}
+
 int threads_share_pools_of_a_full_device()
 {
 	reset(64 * kMB, 64 * kMB);

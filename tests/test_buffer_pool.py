@@ -23,6 +23,6 @@ def lib(tmp_path_factory):
 
 @pytest.mark.parametrize("case", ["spare_of_other_pools_is_given_up", "a_failed_allocation_leaves_nothing_behind",
                                   "a_pool_keeps_its_limit_and_trims_the_oldest",
-                                  "threads_share_pools_of_a_full_device"])
+                                  "large_buffers_take_what_they_ask_for", "threads_share_pools_of_a_full_device"])
 def test_pools(lib, case):
     assert getattr(lib, case)() == 0
