@@ -180,6 +180,20 @@ int option_parallel_draws();                     // 0 automatic, 1 never, 2 wher
 uint32_t option_sampler_limit();                 // 0 (65536) or the rejection-iteration limit of the samplers
 constexpr int kDualThreads = 320;                // threads per CTA with several particles per SM
 constexpr size_t kSmemPerSM = 228 * 1024;        // shared memory per SM (each resident CTA reserves 1 KB)
+
+// Whether MBP proposals queue their draws (sim_fast.cuh) in `queue` bytes beside a chain's state of
+// `smem` bytes: where an SM that runs at most `most` chains at once then takes its `per_sm` chains in
+// no more rounds.  Resident chains count for more than the queue: 608 chains of 120 areas x 2 ages
+// (two per SM, one with the queue) 4.06 ms per proposal column by column, 5.99 ms queued; 304 of
+// 100 x 1 (two rounds of neither) 1.89 and 1.78 ms.
+inline bool chain_queue_fits(size_t smem, size_t queue, int most, int per_sm)
+{
+	auto rounds = [&](size_t bytes) {
+		const int fit = (int)(kSmemPerSM / (bytes + 1024)), n = fit < most ? fit : most;
+		return n > 0 ? (per_sm + n - 1) / n : 1 << 30;
+	};
+	return smem + queue <= 227 * 1024 && rounds(smem + queue) <= rounds(smem);
+}
 int fast_threads();
 int fast_prepare();                              // one-time constant tables of the fast kernel
 int fast_chain_prepare();                        // the same for the MBP-chain variants (mbp_fast.cu)

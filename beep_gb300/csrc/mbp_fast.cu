@@ -4,6 +4,8 @@
 // and means (FP32) of every column, [slot][chain][step][transition][column];
 // the force of infection is formed from the counts every step, so Imap is not
 // stored (INF_UPDATE and INF_DIF_UPDATE give the same map here).
+#include <algorithm>
+
 #include "sim_fast.cuh"
 
 namespace beep {
@@ -35,11 +37,17 @@ int launch_sim_fast_chain(const ModelDev &m, const BatchDev &b_, void *stream)
 	const int nt = b_.nt > 0 ? b_.nt : fast_pick_threads(m);
 	size_t smem = fast_smem_bytes(m, b_.nslots, b_.m_in_smem != 0, b_.nefoi_stage, b_.gstate != nullptr,
 	                              b_.tn_full ? m.T : m.tn_rows, b_.pop_single != 0, b_.tn_smem != 0, nt);
-	// a proposal's draws are queued where the queue fits beside the chain's state (all of an
-	// SM's chains)
+	// a proposal's draws are queued where that leaves the SM its chains at once (320-thread CTAs:
+	// the layout's own number of them)
 	BatchDev b = b_;
-	const size_t queue = chain_queue_bytes(m.T, m.C, nt), share = kSmemPerSM / (nt == kDualThreads ? b.ctas : 1) - 1024;
-	b.ch_queue = b.mode == 1 && !b.simu_all && smem + queue <= share && smem + queue <= 227 * 1024 ? 1 : 0;
+	int dev = 0, sms = 0;
+	cudaError_t ce = cudaGetDevice(&dev);
+	if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+	if (ce != cudaSuccess) return (int)ce;
+	const size_t queue = chain_queue_bytes(m.T, m.C, nt);
+	const bool dual = nt == kDualThreads;
+	const int most = dual ? b.ctas : min_ctas(nt), per_sm = dual ? b.ctas : (b.P + std::max(1, sms) - 1) / std::max(1, sms);
+	b.ch_queue = b.mode == 1 && !b.simu_all && chain_queue_fits(smem, queue, most, per_sm) ? 1 : 0;
 	if (b.ch_queue) smem += queue;
 	if (nt == kDualThreads) return launch_sim_fast_chain_ctas(m, b, smem, stream);
 	if (nt != fast_pick_threads(m)) return (int)cudaErrorInvalidValue;
