@@ -18,15 +18,24 @@ int fast_chain_prepare()
 
 namespace {
 
-template <int NT>
-int launch_chain_nt(const ModelDev &m, const BatchDev &b, size_t smem, cudaStream_t st)
+template <int NT, int Q>
+int launch_chain_q(const ModelDev &m, const BatchDev &b, size_t smem, cudaStream_t st)
 {
-	auto kern = m.G <= 4 ? sim_fast_kernel<NT, 4, false, true> : m.G <= 8 ? sim_fast_kernel<NT, 8, false, true>
-	          : m.G <= 12 ? sim_fast_kernel<NT, 12, false, true> : sim_fast_kernel<NT, 16, false, true>;
+	constexpr int MB = min_ctas(NT);
+	auto kern = m.G <= 4 ? sim_fast_kernel<NT, 4, false, true, MB, kMaxT, false, Q>
+	          : m.G <= 8 ? sim_fast_kernel<NT, 8, false, true, MB, kMaxT, false, Q>
+	          : m.G <= 12 ? sim_fast_kernel<NT, 12, false, true, MB, kMaxT, false, Q>
+	                      : sim_fast_kernel<NT, 16, false, true, MB, kMaxT, false, Q>;
 	cudaError_t e = allow_dynamic_smem(kern, smem);
 	if (e != cudaSuccess) return (int)e;
 	kern<<<b.P, NT, smem, st>>>(m, b);
 	return (int)cudaGetLastError();
+}
+
+template <int NT>
+int launch_chain_nt(const ModelDev &m, const BatchDev &b, size_t smem, cudaStream_t st)
+{
+	return b.ch_queue ? launch_chain_q<NT, kQueueAlways>(m, b, smem, st) : launch_chain_q<NT, kQueueNever>(m, b, smem, st);
 }
 
 }  // namespace

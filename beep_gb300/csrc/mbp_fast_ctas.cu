@@ -7,14 +7,20 @@
 namespace beep {
 namespace {
 
-template <int MG, int MB>
-int launch_mb(const ModelDev &m, const BatchDev &b, size_t smem, cudaStream_t st)
+template <int MG, int MB, int Q>
+int launch_q(const ModelDev &m, const BatchDev &b, size_t smem, cudaStream_t st)
 {
-	auto kern = sim_fast_kernel<kDualThreads, MG, false, true, MB>;
+	auto kern = sim_fast_kernel<kDualThreads, MG, false, true, MB, kMaxT, false, Q>;
 	cudaError_t e = allow_dynamic_smem(kern, smem);
 	if (e != cudaSuccess) return (int)e;
 	kern<<<b.P, kDualThreads, smem, st>>>(m, b);
 	return (int)cudaGetLastError();
+}
+
+template <int MG, int MB>
+int launch_mb(const ModelDev &m, const BatchDev &b, size_t smem, cudaStream_t st)
+{
+	return b.ch_queue ? launch_q<MG, MB, kQueueAlways>(m, b, smem, st) : launch_q<MG, MB, kQueueNever>(m, b, smem, st);
 }
 
 template <int MG>

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) sim_fast_fused_kernel(const 
 		if (it >= f.nitem) break;
 		int k = 0;
 		while (k + 1 < f.nset && it >= f.first[k + 1]) k++;
-		sim_fast_body<kFusedThreads, MG, false, true, kMaxT>(f.m[k], f.b[k], it - f.first[k]);
+		sim_fast_body<kFusedThreads, MG, false, true, kMaxT, false, kQueueByBatch>(f.m[k], f.b[k], it - f.first[k]);
 	}
 }
 

@@ -1179,8 +1179,12 @@ __device__ __forceinline__ int pd_steps(const ModelDev &m, const BatchDev &b, co
 
 // One particle (or MBP chain) p of a batch over its whole step range, run by
 // the NT threads of a CTA.  MT: the most transitions the per-column mean
-// registers hold (kMaxT, or kWideT for models with more transitions).
-template <int NT, int MG, bool TC, bool CH, int MT, bool PD = false>
+// registers hold (kMaxT, or kWideT for models with more transitions).  Q: MBP proposals'
+// draws column by column, queued, or as the batch says (b.ch_queue); compiled apart, since
+// both in one kernel cost the column path registers (700 chains of 70 x 8, three per SM: 5.7
+// instead of 5.4 ms per proposal).
+enum { kQueueNever, kQueueAlways, kQueueByBatch };
+template <int NT, int MG, bool TC, bool CH, int MT, bool PD = false, int Q = kQueueNever>
 __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev &b, const int p)
 {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1259,7 +1263,7 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 		s.red = (float *)take(4 * 2 * (size_t)NT);
 		s.mv = NT == kDualThreads ? (float *)take(4 * (size_t)T * NT) : nullptr;
 		s.dn = PD ? (int32_t *)take(4 * (size_t)C * ncol) : nullptr;
-		s.queue = CH && b.ch_queue ? take(chain_queue_bytes(T, C, NT)) : nullptr;
+		s.queue = Q == kQueueAlways || (Q == kQueueByBatch && b.ch_queue) ? take(chain_queue_bytes(T, C, NT)) : nullptr;
 	}
 	// tensor-core FOI (large models, 640 threads): chunk ring, stacked counts, barriers, tensor memory
 	__shared__ uint64_t tc_bars[2 * tc::kStages + 1];
@@ -1371,8 +1375,8 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 
 		// ---- A: per column (c, dp): NMI, means, draws, next population and infectious count
 		const float d = s.dgeo[sb], omd = 1.f - d;
-		const bool queued = CH && s.queue && cmode == 1 && !b.simu_all;
-		if constexpr (CH) {
+		const bool queued = Q == kQueueAlways || (Q == kQueueByBatch && s.queue);
+		if constexpr (Q != kQueueNever) {
 			if (queued)
 				chain_columns<NT, MG>(m, b, tb, s, p, sett, DrawKey{k0, k1, (uint32_t)sett, stream, lim}, pc, pn, Ic_cur,
 				                      Ic_nxt, be, et, Nm, d, omd, cs_i, cs_p);
@@ -1600,10 +1604,10 @@ __device__ __forceinline__ void sim_fast_body(const ModelDev &m, const BatchDev 
 
 // One CTA per particle (or MBP chain): CTA p runs particle p.  PD: the draws of a step
 // one per (transition, column) thread (small models, fast_parallel_draws).
-template <int NT, int MG, bool TC, bool CH = false, int MB = min_ctas(NT), int MT = kMaxT, bool PD = false>
+template <int NT, int MG, bool TC, bool CH = false, int MB = min_ctas(NT), int MT = kMaxT, bool PD = false, int Q = kQueueNever>
 __global__ void __launch_bounds__(NT, MB) sim_fast_kernel(const ModelDev m, const BatchDev b)
 {
-	sim_fast_body<NT, MG, TC, CH, MT, PD>(m, b, blockIdx.x);
+	sim_fast_body<NT, MG, TC, CH, MT, PD, Q>(m, b, blockIdx.x);
 }
 
 // log k! for k < 32 in this translation unit's constant memory, once (before
