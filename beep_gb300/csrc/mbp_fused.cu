@@ -33,7 +33,7 @@ struct FusedChains {
 // one kernel parameter: within the 32764 bytes a launch takes (CUDA 12.1 and later)
 static_assert(sizeof(FusedChains) <= 32764, "the fused launch descriptor exceeds the kernel parameter limit");
 
-template <int MG>
+template <int MG, int Q>
 __global__ void __launch_bounds__(kFusedThreads, 1) sim_fast_fused_kernel(const __grid_constant__ FusedChains f)
 {
 	__shared__ int item;
@@ -45,8 +45,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1) sim_fast_fused_kernel(const 
 		if (it >= f.nitem) break;
 		int k = 0;
 		while (k + 1 < f.nset && it >= f.first[k + 1]) k++;
-		sim_fast_body<kFusedThreads, MG, false, true, kMaxT, false, kQueueByBatch>(f.m[k], f.b[k], it - f.first[k]);
+		sim_fast_body<kFusedThreads, MG, false, true, kMaxT, false, Q>(f.m[k], f.b[k], it - f.first[k]);
 	}
+}
+
+template <int Q>
+void (*pick_fused(int mg))(const FusedChains)
+{
+	return mg <= 4 ? sim_fast_fused_kernel<4, Q> : mg <= 8 ? sim_fast_fused_kernel<8, Q>
+	     : mg <= 12 ? sim_fast_fused_kernel<12, Q> : sim_fast_fused_kernel<16, Q>;
 }
 
 }  // namespace
@@ -76,6 +83,7 @@ int launch_sim_fast_chain_fused(const ModelDev *m, const BatchDev *b, int n, int
 	f.nset = n;
 	f.counter = counter;
 	size_t smem = 0;
+	bool queued = false;
 	for (int k = 0; k < n; k++) {
 		if (!fused_supported(m[k]) || b[k].mode != 1 || b[k].foi_tc || b[k].batched || !b[k].ch_tn || !b[k].ch_mean_f)
 			return (int)cudaErrorInvalidValue;
@@ -86,11 +94,14 @@ int launch_sim_fast_chain_fused(const ModelDev *m, const BatchDev *b, int n, int
 		const size_t need = fused_smem_bytes(m[k], b[k], mg), queue = chain_queue_bytes(m[k].T, m[k].C, kFusedThreads);
 		f.b[k].ch_queue = need + queue <= 226 * 1024 ? 1 : 0;
 		smem = std::max(smem, need + (f.b[k].ch_queue ? queue : 0));
+		queued |= f.b[k].ch_queue != 0;
 	}
 	f.nitem = f.first[n];
 	if (f.nitem == 0) return 0;
-	auto kern = mg <= 4 ? sim_fast_fused_kernel<4> : mg <= 8 ? sim_fast_fused_kernel<8>
-	          : mg <= 12 ? sim_fast_fused_kernel<12> : sim_fast_fused_kernel<16>;
+	// where no set queues its draws, a kernel of the column path alone: both in one cost it registers
+	// (53 chains of 166 x 3 over 296 steps 6.15 ms, 6.03 ms now); one of the queue alone was the slower
+	// (53 of 350 x 10 over 120 steps 10.0 against 9.7 ms)
+	auto kern = queued ? pick_fused<kQueueByBatch>(mg) : pick_fused<kQueueNever>(mg);
 	cudaError_t e = allow_dynamic_smem(kern, smem);
 	if (e != cudaSuccess) return (int)e;
 	cudaStream_t st = (cudaStream_t)stream;
