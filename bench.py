@@ -379,8 +379,8 @@ def fast_loglik_error(dm, m, tabs, group_of, n: int, seed: int):
 def run_particle_filter(reps: int, seed: int, N: int = 256, section_steps: int = 28):
     """PMCMC likelihood estimates: the bootstrap particle filter of the
     10-area x 3-age workload (dt 0.25, 100 days, 400 steps), N particles, one
-    parameter set, sections of 28 steps with multinomial resampling and the
-    ancestor-state gather on the device between sections.  Estimates per
+    parameter set, sections of 28 steps with multinomial resampling on the
+    device, each section started from its ancestors' states.  Estimates per
     second in both forms (each call is one full estimate: host in, estimate
     out)."""
     from beep_gb300 import capi, model_builder as mb, synth
